@@ -7,6 +7,7 @@ only type of the path, which is forward only.
 """
 import math
 
+import numpy as np
 import torch
 
 from dlprimitives_b200 import capi, hostapi, resnet50
@@ -154,7 +155,11 @@ def prepare(case, seed):
     # the network: built, its weights uploaded; the service hands it one device tensor per request, on its own stream
     net_json = _net_json(case)
     if case["folded"] not in _net_params:
-        _net_params[case["folded"]] = resnet50.make_params(net_json, seed=NET_SEED)
+        # random weights let the activations grow through the residual sums; the classifier is scaled so that its logits have a
+        # trained network's spread (standard deviation about 2) and the softmax is not a one
+        params = resnet50.make_params(net_json, seed=NET_SEED)
+        params["fc.0"] = params["fc.0"] * np.float32(1.0 / 2000)
+        _net_params[case["folded"]] = params
     net = hostapi.Net(net_json)
     for name, value in _net_params[case["folded"]].items():
         net.set_param(name, value)
@@ -234,7 +239,102 @@ def work(case):
 
 def tolerance(case):
     # About four times what the path differs by from itself in 64 bits: single calls rel 2.2e-6, max 1.0e-5; the network's 54
-    # layers carry each other's rounding on: logits rel 5.0e-5, max 5.9e-5.
+    # layers carry each other's rounding on: logits (spread 2) rel 5.0e-5, and the probabilities by as much as the logits differ, 1e-4.
     if case["kind"] == "net":
-        return {"rel": 2e-4, "max": 8e-4}
+        return {"rel": 4e-4, "max": 1.6e-3}
     return {"rel": 1e-5, "max": 5e-5}
+
+
+# ---- the same results in 64 bits, with plain torch ----------------------------------------------------------------------
+
+def _act64(y, act):
+    return y.clamp_(min=0.0) if act == "relu" else (y.clamp_(0.0, 6.0) if act == "relu6" else y)
+
+
+def _conv64(x, w, bias, stride, pad, act="identity"):
+    """A dense convolution as patches times weights, a few images at a time."""
+    n, _, h, wd = x.shape
+    o, _, kh, kw = w.shape
+    oh, ow = (h + 2 * pad - kh) // stride + 1, (wd + 2 * pad - kw) // stride + 1
+    w64 = w.double().reshape(o, -1)
+    y = torch.empty(n, o, oh, ow, dtype=torch.float64, device=x.device)
+    step = max(1, int(2e8 // (w64.shape[1] * oh * ow)))
+    for i in range(0, n, step):
+        part = x[i:i + step].double()
+        if kh == kw == 1:
+            cols = part[:, :, ::stride, ::stride].reshape(part.shape[0], part.shape[1], -1)
+        else:
+            cols = torch.nn.functional.unfold(part, (kh, kw), padding=pad, stride=stride)
+        r = torch.matmul(w64, cols)
+        if bias is not None:
+            r += bias.double()[:, None]
+        y[i:i + step] = _act64(r, act).reshape(part.shape[0], o, oh, ow)
+    return y
+
+
+def _depthwise64(x, w, bias, stride, act):
+    n, c, h, wd = x.shape
+    oh, ow = (h - 1) // stride + 1, (wd - 1) // stride + 1
+    xp = torch.nn.functional.pad(x.double(), (1, 1, 1, 1))
+    y = bias.double()[None, :, None, None].expand(n, c, oh, ow).clone()
+    for i in range(3):
+        for j in range(3):
+            y += w[:, 0, i, j].double()[None, :, None, None] * xp[:, :, i:i + (oh - 1) * stride + 1:stride, j:j + (ow - 1) * stride + 1:stride]
+    return _act64(y, act)
+
+
+def _net64(net_json, params, x):
+    """The network's operators one by one; every parameter and the input are the fp32 values the network has."""
+    p = {name: torch.from_numpy(value).to(x.device) for name, value in params.items()}
+    t = {net_json["inputs"][0]["name"]: x.double()}
+    last = {name: i for i, op in enumerate(net_json["operators"]) for name in op["inputs"]}
+    for i, op in enumerate(net_json["operators"]):
+        o, src, name = op["options"], [t[k] for k in op["inputs"]], op["name"]
+        if op["type"] == "Convolution2D":
+            y = _conv64(src[0], p[name + ".0"], p.get(name + ".1") if o["bias"] else None, o["stride"][0], o["pad"][0], o.get("activation", "identity"))
+        elif op["type"] == "BatchNorm":
+            mean, var, gamma, beta = [p["%s.%d" % (name, k)].double()[None, :, None, None] for k in range(4)]
+            y = (src[0] - mean) / (var + o["eps"]).sqrt() * gamma + beta
+        elif op["type"] == "Activation":
+            y = _act64(src[0].clone(), o["activation"])
+        elif op["type"] == "Pooling2D":
+            y = torch.nn.functional.max_pool2d(src[0], o["kernel"], o["stride"], o["pad"])
+        elif op["type"] == "Elementwise":
+            y = _act64(src[0] + src[1], o["activation"])
+        elif op["type"] == "GlobalPooling":
+            y = src[0].mean(dim=(2, 3))
+        elif op["type"] == "InnerProduct":
+            y = src[0] @ p[name + ".0"].double().t() + p[name + ".1"].double()
+        else:
+            y = torch.softmax(src[0], dim=1)
+        t[op["outputs"][0]] = y
+        for k in op["inputs"]:
+            if last[k] == i and k not in net_json["outputs"]:
+                t.pop(k, None)
+    return t
+
+
+def exact(case, seed):
+    kind = case["kind"]
+    s = prepare(case, seed)
+    if kind == "ip":
+        return _act64(s["x"].double() @ s["w"].double().t() + s["bias"].double(), case["act"])
+    if kind == "gemm":
+        a, b = s["a"].double(), s["b"].double()
+        c = (a.transpose(-1, -2) if case["ta"] else a) @ (b.transpose(-1, -2) if case["tb"] else b)
+        if s["bias"] is not None:
+            c = c + s["bias"].double()
+        return _act64(c, case["act"]).reshape(s["c"].shape)
+    if kind == "conv":
+        y = _conv64(s["x"], s["w"], s["bias"], case["stride"], case["pad"], case["act"])
+        return torch.relu_(y.add_(s["res"])) if case["res"] else y
+    if kind == "block":
+        mid = _depthwise64(s["x"], s["dw_params"][0], s["dw_params"][1], case["stride"], "relu6")
+        return _conv64(mid, s["pw_params"][0], s["pw_params"][1], 1, 0, "relu6")
+    net_json = _net_json(case)
+    fc, prob, step = [], [], 32
+    for i in range(0, case["batch"], step):
+        t = _net64(net_json, _net_params[case["folded"]], s["x"][i:i + step])
+        fc.append(t["fc"])
+        prob.append(t["prob"])
+    return {"fc": torch.cat(fc), "prob": torch.cat(prob)}
