@@ -14,6 +14,7 @@ constexpr int TM = 64, TN = 64, TK = 16, THREADS = 256;
 __global__ void __launch_bounds__(THREADS)
 contraction_ffma_kernel(Contraction p, long long a_group_stride, long long b_group_stride, int out_group_channels, long long y_group_stride)
 {
+    pdl_wait();
     __shared__ float As[TK][TM + 4];
     __shared__ float Bs[TK][TN + 4];
 
@@ -104,8 +105,8 @@ dlp_status launch_contraction_ffma(const Contraction &p, int groups, long long a
     const long long gx = ceil_div<long long>(p.rows, TM);
     if(gx > 0x7fffffffLL) return fail(DLP_INVALID_ARGUMENT, "too many output rows for one launch");
     dim3 grid((unsigned)gx, (unsigned)ceil_div(p.cols, TN), (unsigned)groups);
-    contraction_ffma_kernel<<<grid, THREADS, 0, stream>>>(p, a_group_stride, b_group_stride, out_group_channels, y_group_stride);
-    DLP_LAUNCH_OK("contraction_ffma_kernel");
+    DLP_LAUNCH_PDL(launch_pdl(false, contraction_ffma_kernel, grid, THREADS, 0, stream, p, a_group_stride, b_group_stride,
+                   out_group_channels, y_group_stride), "contraction_ffma_kernel");
     return DLP_OK;
 }
 

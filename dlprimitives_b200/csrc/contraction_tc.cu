@@ -192,6 +192,7 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *(volatile uint32_t *)&sh->tmem_base;
+    pdl_wait();          // everything up to here ran under the kernel before; from here on global memory is read
 
     // ---- epilogue pieces shared by the accumulate warps and, for a CTA's last work item, the loader warps
     // identity / relu / relu6 are a clamp; with no per-row bias and no beta the whole epilogue is
@@ -776,6 +777,7 @@ __global__ void prepack_kernel(const float *__restrict__ b, long long col_stride
                                int n_pad, int k_pad, int bn, int taps, float *__restrict__ packed, long long b_batch_stride, int n_major,
                                int row_kw)
 {
+    pdl_wait();
     const int chunks = k_pad / 4;
     const long long total = (long long)n_pad * chunks;
     b += blockIdx.y * b_batch_stride;           // a batch of matrices: blockIdx.y picks one, packed one after the other
@@ -830,6 +832,7 @@ __global__ void prepack_kernel(const float *__restrict__ b, long long col_stride
 // depend on timing) and apply the epilogue.  Partials are column-major [part][col][rows_pad].
 __global__ void split_finish_kernel(const Contraction p, const float *__restrict__ partial, int splits, long long split_stride, long long rows_pad)
 {
+    pdl_wait();
     const long long total = p.rows * p.cols;
     for(long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
         const int col = int(idx / p.rows);
@@ -862,9 +865,9 @@ dlp_status tc_prepack(const TcPacked &L, const float *b, long long b_col_stride,
     const int threads = 256;
     const int blocks = int(std::min<long long>(ceil_div<long long>(total, threads), 8 * sm_count()));
     if(batch < 1 || batch > 65535) return fail(DLP_INVALID_ARGUMENT, "a batched product takes 1 to 65535 matrices");
-    tc::prepack_kernel<<<dim3(blocks, batch), threads, 0, stream>>>(b, b_col_stride, b_k_stride, cols, k, L.n_pad, L.k_pad, L.bn, taps, packed,
-                                                                    b_batch_stride, b_col_stride == 1 && b_k_stride != 1 ? 1 : 0, row_kw);
-    DLP_LAUNCH_OK("prepack_kernel");
+    DLP_LAUNCH_PDL(launch_pdl(one_wave((long long)blocks * batch, threads), tc::prepack_kernel, dim3(blocks, batch), threads, 0, stream, b,
+                   b_col_stride, b_k_stride, cols, k, L.n_pad, L.k_pad, L.bn, taps, packed, b_batch_stride,
+                   b_col_stride == 1 && b_k_stride != 1 ? 1 : 0, row_kw), "prepack_kernel");
     return DLP_OK;
 }
 
@@ -932,9 +935,9 @@ dlp_status launch_bn(const Contraction &p, const TcPacked &L, const float *packe
 #endif
     int *status = device_status_word();
     if(!status) return fail(DLP_CUDA_ERROR, "cannot resolve the device status word");
-    tc::contraction_tf32x3_kernel<BN, MODE><<<grid, tc::NUM_THREADS, smem, stream>>>(packed, p, L.k_pad / tc::BK / splits, n_tiles, num_tiles,
-                                                                                     splits, split_stride, ktab_entries, status, diag, trace, batch);
-    DLP_LAUNCH_OK("contraction_tf32x3_kernel");
+    DLP_LAUNCH_PDL(launch_pdl(num_tiles * batch.count <= sm_count(), tc::contraction_tf32x3_kernel<BN, MODE>, grid, tc::NUM_THREADS, smem,
+                   stream, packed, p, L.k_pad / tc::BK / splits, n_tiles, num_tiles, splits, split_stride, ktab_entries, status, diag,
+                   trace, batch), "contraction_tf32x3_kernel");
 #ifdef DLP_TC_DIAGNOSTICS
     if(trace) {
         static long long host[64 * 16];
@@ -1005,8 +1008,8 @@ dlp_status launch_contraction_tc(const Contraction &p, const TcPacked &L, const 
     if(st != DLP_OK || splits == 1) return st;
     const long long total = p.rows * p.cols;
     const int blocks = int(std::min<long long>(ceil_div<long long>(total, 256), 16 * sm_count()));
-    tc::split_finish_kernel<<<blocks, 256, 0, stream>>>(p, static_cast<const float *>(scratch), splits, split_stride, rows_pad);
-    DLP_LAUNCH_OK("split_finish_kernel");
+    DLP_LAUNCH_PDL(launch_pdl(one_wave(blocks, 256), tc::split_finish_kernel, blocks, 256, 0, stream, p,
+                   static_cast<const float *>(scratch), splits, split_stride, rows_pad), "split_finish_kernel");
     return DLP_OK;
 }
 

@@ -34,6 +34,7 @@ struct DwParams {
 template<int KS, int ST>
 __global__ void __launch_bounds__(THREADS) depthwise_kernel(DwParams p)
 {
+    pdl_wait();
     __shared__ __align__(16) float tile[SMEM_FLOATS];
     const int ks = KS > 0 ? KS : p.ks;
     const long long plane0 = (long long)(blockIdx.x / p.bands) * p.planes_per_cta;
@@ -186,6 +187,7 @@ __global__ void __launch_bounds__(THREADS) depthwise_kernel(DwParams p)
 template<int S, int V, int RS>
 __global__ void __launch_bounds__(THREADS) depthwise3_reg_kernel(DwParams p, long long groups, int qw, int strips)
 {
+    pdl_wait();
     constexpr int RI = S * (RS - 1) + 3;      // input rows a strip reads
     constexpr int VO = V / S;                 // outputs per lane and row
     const unsigned full = 0xffffffffu;
@@ -266,6 +268,7 @@ __global__ void __launch_bounds__(THREADS) depthwise3_reg_kernel(DwParams p, lon
 template<int W, int S>
 __global__ void __launch_bounds__(THREADS) depthwise3_rows_kernel(DwParams p, long long total_rows)
 {
+    pdl_wait();
     constexpr int OWC = S == 1 ? W : (W + 1) / 2;          // outputs per row
     const unsigned full = 0xffffffffu;
     const long long wid = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
@@ -340,6 +343,7 @@ __global__ void __launch_bounds__(THREADS) depthwise3_rows_kernel(DwParams p, lo
 // U such groups a grid stride apart with their loads issued together; the plane index is a 32-bit division.
 __global__ void __launch_bounds__(THREADS) depthwise1_scale_kernel(DwParams p, unsigned total4, unsigned total, int plane, int vec)
 {
+    pdl_wait();
     constexpr int U = 4;
     const unsigned nthreads = gridDim.x * blockDim.x;
     for(unsigned g0 = blockIdx.x * blockDim.x + threadIdx.x; g0 < total4; g0 += U * nthreads) {
@@ -417,8 +421,8 @@ dlp_status launch_depthwise(const float *x, const float *w, const float *bias, f
         const int plane = H * W;
         const int vec = plane % 4 == 0 && reinterpret_cast<uintptr_t>(y) % 16 == 0;
         const unsigned blocks = std::max(1u, std::min(ceil_div(total4, unsigned(THREADS * 4)), unsigned(16 * sm_count())));
-        depthwise1_scale_kernel<<<blocks, THREADS, 0, stream>>>(p, total4, total, plane, vec);
-        DLP_LAUNCH_OK("depthwise1_scale_kernel");
+        DLP_LAUNCH_PDL(launch_pdl(one_wave(blocks, THREADS), depthwise1_scale_kernel, blocks, THREADS, 0, stream, p, total4, total, plane,
+                       vec), "depthwise1_scale_kernel");
         return DLP_OK;
     }
     // (measured: 1.95 against 1.70 TB/s on the 7x7 rows; on 14x14 planes it is slower than the column kernel below, 1.99 against 2.21)
@@ -427,8 +431,8 @@ dlp_status launch_depthwise(const float *x, const float *w, const float *bias, f
         const long long warps = ceil_div<long long>(total_rows, 30);
         const long long blocks = ceil_div<long long>(warps, THREADS / 32);
         if(blocks > 0x7fffffffLL) return fail(DLP_INVALID_ARGUMENT, "depthwise problem too large for one launch");
-        depthwise3_rows_kernel<7, 1><<<(unsigned)blocks, THREADS, 0, stream>>>(p, total_rows);
-        DLP_LAUNCH_OK("depthwise3_rows_kernel");
+        DLP_LAUNCH_PDL(launch_pdl(one_wave(blocks, THREADS), depthwise3_rows_kernel<7, 1>, (unsigned)blocks, THREADS, 0, stream, p,
+                       total_rows), "depthwise3_rows_kernel");
         return DLP_OK;
     }
     // (measured on the MobileNetV2 rows: odd widths -- 4-byte loads -- and whole 14-row planes as one strip at stride 1
@@ -442,7 +446,8 @@ dlp_status launch_depthwise(const float *x, const float *w, const float *bias, f
         const long long warps = ceil_div<long long>(groups, 32) * strips;
         const long long blocks = ceil_div<long long>(warps, THREADS / 32);
         if(blocks > 0x7fffffffLL) return fail(DLP_INVALID_ARGUMENT, "depthwise problem too large for one launch");
-#define DLP_DW_REG(S, V, RS) depthwise3_reg_kernel<S, V, RS><<<(unsigned)blocks, THREADS, 0, stream>>>(p, groups, qw, strips)
+#define DLP_DW_REG(S, V, RS) launched = launch_pdl(one_wave(blocks, THREADS), depthwise3_reg_kernel<S, V, RS>, (unsigned)blocks, THREADS, 0, stream, p, groups, qw, strips)
+        cudaError_t launched;
         switch(stride * 1000 + v * 100 + rs) {
         case 1406: DLP_DW_REG(1, 4, 6); break;
         case 1206: DLP_DW_REG(1, 2, 6); break;
@@ -452,7 +457,7 @@ dlp_status launch_depthwise(const float *x, const float *w, const float *bias, f
         default: DLP_DW_REG(2, 2, 7); break;
         }
 #undef DLP_DW_REG
-        DLP_LAUNCH_OK("depthwise3_reg_kernel");
+        DLP_LAUNCH_PDL(launched, "depthwise3_reg_kernel");
         return DLP_OK;
     }
     const long long plane_elems = (long long)H * W;
@@ -475,14 +480,15 @@ dlp_status launch_depthwise(const float *x, const float *w, const float *bias, f
     }
     const long long blocks = ceil_div<long long>(p.planes, p.planes_per_cta) * p.bands;
     if(blocks > 0x7fffffffLL) return fail(DLP_INVALID_ARGUMENT, "depthwise problem too large for one launch");
+    cudaError_t launched;
     switch(ks * 10 + stride) {
-    case 31: depthwise_kernel<3, 1><<<(unsigned)blocks, THREADS, 0, stream>>>(p); break;
-    case 32: depthwise_kernel<3, 2><<<(unsigned)blocks, THREADS, 0, stream>>>(p); break;
-    case 51: depthwise_kernel<5, 1><<<(unsigned)blocks, THREADS, 0, stream>>>(p); break;
-    case 52: depthwise_kernel<5, 2><<<(unsigned)blocks, THREADS, 0, stream>>>(p); break;
-    default: depthwise_kernel<0, 0><<<(unsigned)blocks, THREADS, 0, stream>>>(p); break;
+    case 31: launched = launch_pdl(one_wave(blocks, THREADS), depthwise_kernel<3, 1>, (unsigned)blocks, THREADS, 0, stream, p); break;
+    case 32: launched = launch_pdl(one_wave(blocks, THREADS), depthwise_kernel<3, 2>, (unsigned)blocks, THREADS, 0, stream, p); break;
+    case 51: launched = launch_pdl(one_wave(blocks, THREADS), depthwise_kernel<5, 1>, (unsigned)blocks, THREADS, 0, stream, p); break;
+    case 52: launched = launch_pdl(one_wave(blocks, THREADS), depthwise_kernel<5, 2>, (unsigned)blocks, THREADS, 0, stream, p); break;
+    default: launched = launch_pdl(one_wave(blocks, THREADS), depthwise_kernel<0, 0>, (unsigned)blocks, THREADS, 0, stream, p); break;
     }
-    DLP_LAUNCH_OK("depthwise_kernel");
+    DLP_LAUNCH_PDL(launched, "depthwise_kernel");
     return DLP_OK;
 }
 

@@ -10,6 +10,7 @@ namespace {
 __global__ void pooling2d_kernel(const float *__restrict__ x, float *__restrict__ y, long long total, int in_h, int in_w, int out_h,
                                  int out_w, int kh, int kw, int sh, int sw, int ph, int pw, int mode_avg, int include_pad)
 {
+    pdl_wait();
     for(long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const int oc = int(i % out_w);
         const long long t = i / out_w;
@@ -47,6 +48,7 @@ __global__ void pooling2d_band_kernel(const float *__restrict__ x, float *__rest
                                       int band_rows, int in_h, int in_w, int out_h, int out_w, int kh_, int kw_, int sh_, int sw_, int ph,
                                       int pw, int mode_avg, int include_pad, int vec_ok)
 {
+    pdl_wait();
     const int kh = K ? K : kh_, kw = K ? K : kw_, sh = S ? S : sh_, sw = S ? S : sw_;
     extern __shared__ float tile[];
     for(long long band = blockIdx.x; band < bands_total; band += gridDim.x) {
@@ -116,6 +118,7 @@ template<int RS>
 __global__ void __launch_bounds__(256) pool_max3s2_kernel(const float *__restrict__ x, float *__restrict__ y, long long items, int col_blocks,
                                                           int strips, int in_h, int in_w, int out_h, int out_w)
 {
+    pdl_wait();
     const long long item = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if(item >= items) return;
@@ -155,6 +158,7 @@ __global__ void __launch_bounds__(256) pool_max3s2_kernel(const float *__restric
 __global__ void __launch_bounds__(128) global_pooling_tile_kernel(const float *__restrict__ x, float *__restrict__ y, int planes, int plane_size,
                                                                   int mode_avg)
 {
+    pdl_wait();
     extern __shared__ float tile[];
     const int plane0 = blockIdx.x * 128, count = min(128, planes - plane0) * plane_size;
     const float *src = x + (long long)plane0 * plane_size;           // 128 * plane_size * 4 bytes per CTA: 16-byte aligned when x is
@@ -173,6 +177,7 @@ __global__ void __launch_bounds__(128) global_pooling_tile_kernel(const float *_
 // one warp per plane
 __global__ void global_pooling_kernel(const float *__restrict__ x, float *__restrict__ y, int planes, int plane_size, int mode_avg)
 {
+    pdl_wait();
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if(warp >= planes) return;
     const float *src = x + (long long)warp * plane_size;
@@ -198,6 +203,7 @@ __device__ __forceinline__ float eltwise_op(float a, float b, int op, float c0, 
 // c may be a or b (in-place Elementwise): no __restrict__ and no non-coherent loads on the operands
 __global__ void elementwise_kernel(const float *a, const float *b, float *c, size_t count, int op, float c0, float c1, int act, int vec_ok)
 {
+    pdl_wait();
     const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
     if(vec_ok) {
         const size_t n4 = count / 4;
@@ -219,6 +225,7 @@ __global__ void elementwise_kernel(const float *a, const float *b, float *c, siz
 // y may be x (in place)
 __global__ void activation_kernel(const float *x, float *y, size_t count, int act)
 {
+    pdl_wait();
     for(size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x)
         y[i] = apply_act(x[i], act);
 }
@@ -226,6 +233,7 @@ __global__ void activation_kernel(const float *x, float *y, size_t count, int ac
 // one CTA per (row, inner) slice; classes strided by `inner`
 __global__ void softmax_kernel(const float *x, float *y, int classes, int inner, int log_mode)
 {
+    pdl_wait();
     __shared__ float red[32];
     const long long slice = blockIdx.x;
     const long long base = (slice / inner) * (long long)classes * inner + slice % inner;
@@ -259,6 +267,7 @@ __global__ void batchnorm_inference_kernel(const float *x, float *y, size_t coun
                                            float eps, const float *__restrict__ mean, const float *__restrict__ var,
                                            const float *__restrict__ gamma, const float *__restrict__ beta)
 {
+    pdl_wait();
     for(size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x) {
         const int f = int((i / plane) % features);
         float a = 1.0f / sqrtf(var[f] + eps);
@@ -315,9 +324,8 @@ dlp_status dlp_pooling2d_fwd(const float *x, float *y, int planes, int in_h, int
         constexpr int RS = 4;      // 4-row strips: measured faster than 8 (fewer registers, more warps in flight)
         const int col_blocks = ceil_div(ow, 32), strips = ceil_div(oh, RS);
         const long long items = (long long)planes * col_blocks * strips;
-        pool_max3s2_kernel<RS><<<unsigned(ceil_div<long long>(items, 8)), 256, 0, (cudaStream_t)stream>>>(x, y, items, col_blocks, strips, in_h, in_w,
-                                                                                                         oh, ow);
-        DLP_LAUNCH_OK("pool_max3s2_kernel");
+        DLP_LAUNCH_PDL(launch_pdl(one_wave(ceil_div<long long>(items, 8), 256), pool_max3s2_kernel<RS>, unsigned(ceil_div<long long>(items,
+                       8)), 256, 0, (cudaStream_t)stream, x, y, items, col_blocks, strips, in_h, in_w, oh, ow), "pool_max3s2_kernel");
         return DLP_OK;
     }
     // Bands of output rows through shared memory when a useful band fits in 12 KB: each input byte is read
@@ -334,21 +342,21 @@ dlp_status dlp_pooling2d_fwd(const float *x, float *y, int planes, int in_h, int
             const int vec_ok = in_w % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0;
             const int grid = int(std::min<long long>(bands_total, (long long)sm_count() * 16));
             const bool square = kernel[0] == kernel[1] && stride[0] == stride[1];
-#define DLP_POOL_BAND(K, S) pooling2d_band_kernel<K, S><<<grid, 256, smem, (cudaStream_t)stream>>>(x, y, bands_total, bands_per_plane, band_rows, \
-            in_h, in_w, oh, ow, kernel[0], kernel[1], stride[0], stride[1], pad[0], pad[1], mode, count_include_pad, vec_ok)
+            cudaError_t launched;
+#define DLP_POOL_BAND(K, S) launched = launch_pdl(one_wave(grid, 256), pooling2d_band_kernel<K, S>, grid, 256, smem, (cudaStream_t)stream, x, y, bands_total, \
+            bands_per_plane, band_rows, in_h, in_w, oh, ow, kernel[0], kernel[1], stride[0], stride[1], pad[0], pad[1], mode, count_include_pad, vec_ok)
             if(square && kernel[0] == 3 && stride[0] == 2) DLP_POOL_BAND(3, 2);
             else if(square && kernel[0] == 2 && stride[0] == 2) DLP_POOL_BAND(2, 2);
             else if(square && kernel[0] == 3 && stride[0] == 1) DLP_POOL_BAND(3, 1);
             else DLP_POOL_BAND(0, 0);
 #undef DLP_POOL_BAND
-            DLP_LAUNCH_OK("pooling2d_band_kernel");
+            DLP_LAUNCH_PDL(launched, "pooling2d_band_kernel");
             return DLP_OK;
         }
     }
-    pooling2d_kernel<<<grid_for(size_t(total), 256), 256, 0, (cudaStream_t)stream>>>(x, y, total, in_h, in_w, oh, ow, kernel[0], kernel[1],
-                                                                                      stride[0], stride[1], pad[0], pad[1], mode,
-                                                                                      count_include_pad);
-    DLP_LAUNCH_OK("pooling2d_kernel");
+    DLP_LAUNCH_PDL(launch_pdl(one_wave(grid_for(size_t(total), 256), 256), pooling2d_kernel, grid_for(size_t(total), 256), 256, 0,
+                   (cudaStream_t)stream, x, y, total, in_h, in_w, oh, ow, kernel[0], kernel[1], stride[0], stride[1], pad[0], pad[1], mode,
+                   count_include_pad), "pooling2d_kernel");
     return DLP_OK;
 }
 
@@ -358,14 +366,14 @@ dlp_status dlp_global_pooling_fwd(const float *x, float *y, int planes, int plan
     DLP_REQUIRE(plane_size > 0 && (mode == 0 || mode == 1), "bad global pooling arguments");
     if(planes <= 0) return DLP_OK;
     if(plane_size % 2 == 1 && plane_size <= 95 && reinterpret_cast<uintptr_t>(x) % 16 == 0) {
-        global_pooling_tile_kernel<<<ceil_div(planes, 128), 128, size_t(128) * plane_size * sizeof(float), (cudaStream_t)stream>>>(x, y, planes,
-                                                                                                                                plane_size, mode);
-        DLP_LAUNCH_OK("global_pooling_tile_kernel");
+        DLP_LAUNCH_PDL(launch_pdl(one_wave(ceil_div(planes, 128), 128), global_pooling_tile_kernel, ceil_div(planes, 128), 128,
+                       size_t(128) * plane_size * sizeof(float), (cudaStream_t)stream, x, y, planes, plane_size, mode),
+                       "global_pooling_tile_kernel");
         return DLP_OK;
     }
     const int threads = 256, warps_per_block = threads / 32;
-    global_pooling_kernel<<<ceil_div(planes, warps_per_block), threads, 0, (cudaStream_t)stream>>>(x, y, planes, plane_size, mode);
-    DLP_LAUNCH_OK("global_pooling_kernel");
+    DLP_LAUNCH_PDL(launch_pdl(one_wave(ceil_div(planes, warps_per_block), threads), global_pooling_kernel, ceil_div(planes,
+                   warps_per_block), threads, 0, (cudaStream_t)stream, x, y, planes, plane_size, mode), "global_pooling_kernel");
     return DLP_OK;
 }
 
@@ -376,8 +384,8 @@ dlp_status dlp_elementwise_fwd(const float *a, const float *b, float *c, size_t 
     DLP_REQUIRE(op >= 0 && op <= 2, "op must be 0 (sum), 1 (prod) or 2 (max)");
     if(count == 0) return DLP_OK;
     const int vec_ok = ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) % 16) == 0;
-    elementwise_kernel<<<grid_for(count / 4 + 1, 256), 256, 0, (cudaStream_t)stream>>>(a, b, c, count, op, coef1, coef2, activation, vec_ok);
-    DLP_LAUNCH_OK("elementwise_kernel");
+    DLP_LAUNCH_PDL(launch_pdl(one_wave(grid_for(count / 4 + 1, 256), 256), elementwise_kernel, grid_for(count / 4 + 1, 256), 256, 0,
+                   (cudaStream_t)stream, a, b, c, count, op, coef1, coef2, activation, vec_ok), "elementwise_kernel");
     return DLP_OK;
 }
 
@@ -385,8 +393,8 @@ dlp_status dlp_activation_fwd(const float *x, float *y, size_t count, int activa
 {
     DLP_REQUIRE(x && y, "null tensor");
     if(count == 0) return DLP_OK;
-    activation_kernel<<<grid_for(count, 256), 256, 0, (cudaStream_t)stream>>>(x, y, count, activation);
-    DLP_LAUNCH_OK("activation_kernel");
+    DLP_LAUNCH_PDL(launch_pdl(one_wave(grid_for(count, 256), 256), activation_kernel, grid_for(count, 256), 256, 0, (cudaStream_t)stream, x,
+                   y, count, activation), "activation_kernel");
     return DLP_OK;
 }
 
@@ -396,8 +404,8 @@ dlp_status dlp_softmax_fwd(const float *x, float *y, int rows, int classes, int 
     DLP_REQUIRE(classes > 0 && inner > 0, "bad softmax shape");
     if(rows <= 0) return DLP_OK;
     const int threads = classes >= 512 ? 256 : (classes >= 128 ? 128 : 32);
-    softmax_kernel<<<(unsigned)((long long)rows * inner), threads, 0, (cudaStream_t)stream>>>(x, y, classes, inner, log_mode);
-    DLP_LAUNCH_OK("softmax_kernel");
+    DLP_LAUNCH_PDL(launch_pdl(one_wave(((long long)rows * inner), threads), softmax_kernel, (unsigned)((long long)rows * inner), threads, 0,
+                   (cudaStream_t)stream, x, y, classes, inner, log_mode), "softmax_kernel");
     return DLP_OK;
 }
 
@@ -408,8 +416,8 @@ dlp_status dlp_batchnorm_inference_fwd(const float *x, float *y, int batch, int 
     DLP_REQUIRE(features > 0 && plane > 0, "bad batch-norm shape");
     const size_t count = size_t(batch) * features * plane;
     if(count == 0) return DLP_OK;
-    batchnorm_inference_kernel<<<grid_for(count, 256), 256, 0, (cudaStream_t)stream>>>(x, y, count, features, plane, eps, mean, var, gamma, beta);
-    DLP_LAUNCH_OK("batchnorm_inference_kernel");
+    DLP_LAUNCH_PDL(launch_pdl(one_wave(grid_for(count, 256), 256), batchnorm_inference_kernel, grid_for(count, 256), 256, 0,
+                   (cudaStream_t)stream, x, y, count, features, plane, eps, mean, var, gamma, beta), "batchnorm_inference_kernel");
     return DLP_OK;
 }
 

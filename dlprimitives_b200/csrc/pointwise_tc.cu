@@ -164,6 +164,7 @@ pointwise_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *(volatile uint32_t *)&sh->tmem_base;
+    pdl_wait();          // everything up to here ran under the kernel before; from here on global memory is read
 
     if(warp == WARP_B) {
         // ------------------------------------------------------------------ B copies
@@ -543,8 +544,8 @@ static dlp_status launch_bn(const CUtensorMap &tx, const CUtensorMap &ty, const 
         r.e_bufs = std::min(MAX_E_BUFS, avail - r.s_stages);
     }
     const int smem_bytes = SMEM_FIXED + r.b_bytes + (r.s_stages + r.e_bufs) * A_STAGE_BYTES;
-    pointwise_tf32x3_kernel<BN><<<grid, NUM_THREADS, smem_bytes, stream>>>(tx, ty, tr, packed, r, status);
-    DLP_LAUNCH_OK("pointwise_tf32x3_kernel");
+    DLP_LAUNCH_PDL(launch_pdl(q.num_items <= sm_count(), pointwise_tf32x3_kernel<BN>, grid, NUM_THREADS, smem_bytes, stream, tx, ty, tr,
+                   packed, r, status), "pointwise_tf32x3_kernel");
     return DLP_OK;
 }
 

@@ -187,6 +187,7 @@ staged_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *(volatile uint32_t *)&sh->tmem_base;
+    pdl_wait();          // everything up to here ran under the kernel before; from here on global memory is read
 
     if(warp == WARP_A) {
         // ------------------------------------------------------------------ patch copies
@@ -576,8 +577,8 @@ static dlp_status launch_bn(const CUtensorMap &tx, const CUtensorMap &ty, const 
     r.s_stages = std::min(MAX_S_STAGES, left / r.slot_bytes);
     if(r.s_stages < 2) return fail(DLP_INVALID_ARGUMENT, "no room for two input patches");
     const int smem_bytes = SMEM_FIXED + r.b_bytes + r.s_stages * r.slot_bytes + r.e_bufs * E_BUF_BYTES;
-    staged_tf32x3_kernel<BN><<<grid, NUM_THREADS, smem_bytes, stream>>>(tx, ty, packed, r, status);
-    DLP_LAUNCH_OK("staged_tf32x3_kernel");
+    DLP_LAUNCH_PDL(launch_pdl(q.num_items <= sm_count(), staged_tf32x3_kernel<BN>, grid, NUM_THREADS, smem_bytes, stream, tx, ty, packed, r,
+                   status), "staged_tf32x3_kernel");
     return DLP_OK;
 }
 

@@ -27,6 +27,7 @@ constexpr int WTHREADS = 256;
 // U[xi][c][o] = (G g G^T)[xi] for filter (o, c); o padded to cout_pad with zeros
 __global__ void winograd_filter_transform_kernel(const float *__restrict__ w, float *__restrict__ u, int cin, int cout, int cout_pad)
 {
+    pdl_wait();
     const long long total = (long long)cin * cout_pad;
     for(long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
         const int c = int(idx / cout_pad), o = int(idx - (long long)c * cout_pad);
@@ -67,6 +68,7 @@ struct WinogradArgs {
 __global__ void __launch_bounds__(WTHREADS)
 winograd_f23_kernel(const WinogradArgs a)
 {
+    pdl_wait();
     __shared__ float Vs[16][WC][WT];
     __shared__ float Us[16][WC][WF];
 
@@ -199,8 +201,8 @@ dlp_status winograd_filter_transform(const float *w, float *u, int cin, int cout
     const int cout_pad = round_up(cout, WF);
     const long long total = (long long)cin * cout_pad;
     const int blocks = int(std::min<long long>(ceil_div<long long>(total, 256), 8 * sm_count()));
-    winograd_filter_transform_kernel<<<blocks, 256, 0, stream>>>(w, u, cin, cout, cout_pad);
-    DLP_LAUNCH_OK("winograd_filter_transform_kernel");
+    DLP_LAUNCH_PDL(launch_pdl(one_wave(blocks, 256), winograd_filter_transform_kernel, blocks, 256, 0, stream, w, u, cin, cout, cout_pad),
+                   "winograd_filter_transform_kernel");
     return DLP_OK;
 }
 
@@ -217,8 +219,7 @@ dlp_status launch_winograd_f23(const float *x, const float *u, const float *bias
     const long long gx = ceil_div<long long>(a.tiles, WT);
     if(gx > 0x7fffffffLL) return fail(DLP_INVALID_ARGUMENT, "too many output tiles for one launch");
     dim3 grid((unsigned)gx, (unsigned)(a.cout_pad / WF));
-    winograd_f23_kernel<<<grid, WTHREADS, 0, stream>>>(a);
-    DLP_LAUNCH_OK("winograd_f23_kernel");
+    DLP_LAUNCH_PDL(launch_pdl(false, winograd_f23_kernel, grid, WTHREADS, 0, stream, a), "winograd_f23_kernel");
     return DLP_OK;
 }
 

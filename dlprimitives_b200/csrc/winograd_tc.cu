@@ -24,6 +24,7 @@ namespace {
 // Uraw[xi][o][c] = (G g G^T)[xi] for filter (o, c)
 __global__ void wtc_filter_kernel(const float *__restrict__ w, float *__restrict__ u, int cin, int cout)
 {
+    pdl_wait();
     const long long total = (long long)cin * cout;
     for(long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
         float g[3][3];
@@ -54,6 +55,7 @@ struct Geometry {
 // one thread per (channel plane, tile): reads the 4x4 patch, writes the 16 transformed values (tiles contiguous across lanes)
 __global__ void wtc_input_kernel(const float *__restrict__ x, float *__restrict__ v, Geometry q)
 {
+    pdl_wait();
     const long long per_image = (long long)q.tiles_h * q.tiles_w;
     const long long total = q.tiles * q.cin;
     for(long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
@@ -102,6 +104,7 @@ struct OutArgs {
 // one thread per (output channel plane, tile): reads the 16 products, writes the 2x2 outputs
 __global__ void wtc_output_kernel(const float *__restrict__ mm, Geometry q, OutArgs a)
 {
+    pdl_wait();
     const long long per_image = (long long)q.tiles_h * q.tiles_w;
     const long long total = q.tiles * q.cout;
     for(long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
@@ -170,8 +173,7 @@ dlp_status winograd_tc_filter_transform(const float *w, float *packed, int cin, 
     float *raw = packed + 16 * (L.bytes() / sizeof(float));
     const long long total = (long long)cin * cout;
     const int blocks = int(std::min<long long>(ceil_div<long long>(total, 256), 8 * sm_count()));
-    wtc_filter_kernel<<<blocks, 256, 0, stream>>>(w, raw, cin, cout);
-    DLP_LAUNCH_OK("wtc_filter_kernel");
+    DLP_LAUNCH_PDL(launch_pdl(one_wave(blocks, 256), wtc_filter_kernel, blocks, 256, 0, stream, w, raw, cin, cout), "wtc_filter_kernel");
     return tc_prepack(L, raw, cin, 1, cout, cin, packed, 0, stream, 16, total);
 }
 
@@ -187,8 +189,7 @@ dlp_status launch_winograd_tc(const float *x, const float *packed, const float *
     float *v = static_cast<float *>(ws);
     float *mm = v + 16ll * q.tiles_pad * cin;
     const int blocks = int(std::min<long long>(ceil_div<long long>(q.tiles * std::max(cin, cout), 256), 32ll * sm_count()));
-    wtc_input_kernel<<<blocks, 256, 0, stream>>>(x, v, q);
-    DLP_LAUNCH_OK("wtc_input_kernel");
+    DLP_LAUNCH_PDL(launch_pdl(one_wave(blocks, 256), wtc_input_kernel, blocks, 256, 0, stream, x, v, q), "wtc_input_kernel");
 
     Contraction p;
     memset(&p, 0, sizeof(p));
@@ -212,8 +213,7 @@ dlp_status launch_winograd_tc(const float *x, const float *packed, const float *
 
     OutArgs a;
     a.bias = bias; a.residual = residual; a.y = y; a.act = act; a.post_act = post_act; a.factor = factor; a.residual_scale = residual_scale;
-    wtc_output_kernel<<<blocks, 256, 0, stream>>>(mm, q, a);
-    DLP_LAUNCH_OK("wtc_output_kernel");
+    DLP_LAUNCH_PDL(launch_pdl(one_wave(blocks, 256), wtc_output_kernel, blocks, 256, 0, stream, mm, q, a), "wtc_output_kernel");
     return DLP_OK;
 }
 
