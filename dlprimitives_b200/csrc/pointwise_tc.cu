@@ -540,7 +540,11 @@ static dlp_status launch_bn(const CUtensorMap &tx, const CUtensorMap &ty, const 
         r.e_bufs = avail - r.s_stages;
     }
     else {
-        r.s_stages = std::min(MAX_S_STAGES - 1, avail / 2);
+        // An even number: the two converter groups take the k-blocks in turn, and with an odd one a group would meet ring entries
+        // whose last copy was the other group's.  A wait tells two successive copies of an entry apart only by one parity bit, so
+        // while that copy is still on its way the entry passes for filled: the group reads it too early, hands it back a
+        // second time, and from then on copies land in entries that are being read -- or after the block has left.
+        r.s_stages = (std::min(MAX_S_STAGES - 1, avail / 2) + 1) & ~1;
         r.e_bufs = std::min(MAX_E_BUFS, avail - r.s_stages);
     }
     const int smem_bytes = SMEM_FIXED + r.b_bytes + (r.s_stages + r.e_bufs) * A_STAGE_BYTES;
