@@ -69,6 +69,8 @@ inline cudaError_t launch_pdl(bool early, void (*kernel)(P...), dim3 grid, dim3 
 
 // blocks of a plain kernel (threads each, little shared memory) that are all resident at once
 inline bool one_wave(long long blocks, int threads) { return blocks * threads <= (long long)sm_count() * 2048; }
+// work items of a persistent tensor-core kernel that are few enough for the set-up to matter
+inline bool few_items(long long items) { return items <= 4ll * sm_count(); }
 
 // ---- device side ---------------------------------------------------------------------------------
 // Activation definitions shared by every epilogue; they follow the reference's device macros

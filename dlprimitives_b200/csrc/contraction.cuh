@@ -168,6 +168,13 @@ dlp_status launch_pointwise_tc(const Contraction &p, const TcPacked &L, const fl
 bool staged_tc_eligible(const Contraction &p, const TcPacked &L);
 dlp_status launch_staged_tc(const Contraction &p, const TcPacked &L, const float *packed, cudaStream_t stream);
 
+// Matrices and stride-1 convolutions whose rows and planes the copy engines can address (16-byte pitches), with any K
+// (stream_tc.cu).  splits: parts of K as work items of their own, part s writing to y + s * split_stride.
+// launch_contraction_tc hands eligible problems over by itself.
+bool stream_tc_eligible(const Contraction &p, const TcPacked &L, int splits, const TcBatch &batch);
+dlp_status launch_stream_tc(const Contraction &p, const TcPacked &L, const float *packed, cudaStream_t stream, int splits, long long split_stride,
+                            const TcBatch &batch);
+
 // Winograd F(2x2, 3x3), stride 1, padding 1 (winograd.cu).  u: the transformed filters, winograd_packed_bytes() long.
 size_t winograd_packed_bytes(int cin, int cout);
 dlp_status winograd_filter_transform(const float *w, float *u, int cin, int cout, cudaStream_t stream);

@@ -935,7 +935,7 @@ dlp_status launch_bn(const Contraction &p, const TcPacked &L, const float *packe
 #endif
     int *status = device_status_word();
     if(!status) return fail(DLP_CUDA_ERROR, "cannot resolve the device status word");
-    DLP_LAUNCH_PDL(launch_pdl(num_tiles * batch.count <= sm_count(), tc::contraction_tf32x3_kernel<BN, MODE>, grid, tc::NUM_THREADS, smem,
+    DLP_LAUNCH_PDL(launch_pdl(few_items(num_tiles * batch.count), tc::contraction_tf32x3_kernel<BN, MODE>, grid, tc::NUM_THREADS, smem,
                    stream, packed, p, L.k_pad / tc::BK / splits, n_tiles, num_tiles, splits, split_stride, ktab_entries, status, diag,
                    trace, batch), "contraction_tf32x3_kernel");
 #ifdef DLP_TC_DIAGNOSTICS
@@ -990,7 +990,8 @@ dlp_status launch_contraction_tc(const Contraction &p, const TcPacked &L, const 
         q.residual = nullptr;
     }
     dlp_status st = DLP_INVALID_ARGUMENT;
-    switch(L.bn * 4 + p.a_mode) {
+    if(stream_tc_eligible(q, L, splits, batch)) st = launch_stream_tc(q, L, packed, stream, splits, split_stride, batch);
+    else switch(L.bn * 4 + p.a_mode) {
     case 32 * 4 + A_GATHER: st = launch_bn<32, A_GATHER>(q, L, packed, stream, splits, split_stride, batch); break;
     case 32 * 4 + A_STRIDED: st = launch_bn<32, A_STRIDED>(q, L, packed, stream, splits, split_stride, batch); break;
     case 32 * 4 + A_TAPBLOCK: st = launch_bn<32, A_TAPBLOCK>(q, L, packed, stream, splits, split_stride, batch); break;

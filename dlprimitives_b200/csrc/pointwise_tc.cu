@@ -548,7 +548,7 @@ static dlp_status launch_bn(const CUtensorMap &tx, const CUtensorMap &ty, const 
         r.e_bufs = std::min(MAX_E_BUFS, avail - r.s_stages);
     }
     const int smem_bytes = SMEM_FIXED + r.b_bytes + (r.s_stages + r.e_bufs) * A_STAGE_BYTES;
-    DLP_LAUNCH_PDL(launch_pdl(q.num_items <= sm_count(), pointwise_tf32x3_kernel<BN>, grid, NUM_THREADS, smem_bytes, stream, tx, ty, tr,
+    DLP_LAUNCH_PDL(launch_pdl(few_items(q.num_items), pointwise_tf32x3_kernel<BN>, grid, NUM_THREADS, smem_bytes, stream, tx, ty, tr,
                    packed, r, status), "pointwise_tf32x3_kernel");
     return DLP_OK;
 }

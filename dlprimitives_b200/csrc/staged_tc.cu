@@ -577,7 +577,7 @@ static dlp_status launch_bn(const CUtensorMap &tx, const CUtensorMap &ty, const 
     r.s_stages = std::min(MAX_S_STAGES, left / r.slot_bytes);
     if(r.s_stages < 2) return fail(DLP_INVALID_ARGUMENT, "no room for two input patches");
     const int smem_bytes = SMEM_FIXED + r.b_bytes + r.s_stages * r.slot_bytes + r.e_bufs * E_BUF_BYTES;
-    DLP_LAUNCH_PDL(launch_pdl(q.num_items <= sm_count(), staged_tf32x3_kernel<BN>, grid, NUM_THREADS, smem_bytes, stream, tx, ty, packed, r,
+    DLP_LAUNCH_PDL(launch_pdl(few_items(q.num_items), staged_tf32x3_kernel<BN>, grid, NUM_THREADS, smem_bytes, stream, tx, ty, packed, r,
                    status), "staged_tf32x3_kernel");
     return DLP_OK;
 }

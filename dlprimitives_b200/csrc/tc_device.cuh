@@ -14,10 +14,11 @@ __device__ __forceinline__ void mbar_init(unsigned long long *bar, uint32_t coun
 {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
 }
-__device__ __forceinline__ void mbar_arrive(unsigned long long *bar)
+__device__ __forceinline__ void mbar_arrive(uint32_t bar)
 {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(unsigned long long *bar) { mbar_arrive(smem_u32(bar)); }
 __device__ __forceinline__ void mbar_arrive_expect_tx(unsigned long long *bar, uint32_t bytes)
 {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
@@ -51,7 +52,14 @@ __device__ __forceinline__ long long global_ns()
 }
 // Bounded wait by one thread.  Returns false when the CTA is aborting or the time limit ran out
 // (then it raises the abort).
-static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, int *abort_flag, int *status, int code)
+// (Out of line, since the roles of a kernel share a small instruction cache -- except in a kernel that moves registers between
+// its warpgroups, where a call has no register count to agree on: such a file defines DLP_INLINE_WAITS.)
+#ifdef DLP_INLINE_WAITS
+#define DLP_WAIT_INLINING __forceinline__
+#else
+#define DLP_WAIT_INLINING __noinline__
+#endif
+static __device__ DLP_WAIT_INLINING bool mbar_wait_slow(uint32_t bar, uint32_t parity, int *abort_flag, int *status, int code)
 {
     #pragma unroll 1
     for(int i = 0; i < 32; i++)
@@ -81,7 +89,8 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, uint32_t pari
     return mbar_wait(smem_u32(bar), parity, abort_flag, status, code);
 }
 // The same for a whole warp: one lane polls (32 lanes polling one barrier serialise), all get the answer.
-__device__ __forceinline__ bool warp_wait(unsigned long long *bar, uint32_t parity, int *abort_flag, int *status, int code, int lane)
+template<typename Bar>
+__device__ __forceinline__ bool warp_wait(Bar bar, uint32_t parity, int *abort_flag, int *status, int code, int lane)
 {
     int ok = 1;
     __syncwarp();
@@ -196,7 +205,7 @@ __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&v)[32])
                    "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
                  : "r"(taddr) : "memory");
 }
-__device__ __forceinline__ bool act_is_clamp(int act) { return act == DLP_ACT_IDENTITY || act == DLP_ACT_RELU || act == DLP_ACT_RELU6; }
+__host__ __device__ __forceinline__ bool act_is_clamp(int act) { return act == DLP_ACT_IDENTITY || act == DLP_ACT_RELU || act == DLP_ACT_RELU6; }
 __device__ __forceinline__ float2 act_clamp(int act)
 {
     return make_float2(act == DLP_ACT_IDENTITY ? -INFINITY : 0.0f, act == DLP_ACT_RELU6 ? 6.0f : INFINITY);
