@@ -222,12 +222,25 @@ __global__ void elementwise_kernel(const float *a, const float *b, float *c, siz
         for(size_t i = tid; i < count; i += step) c[i] = apply_act(eltwise_op(a[i], b[i], op, c0, c1), act);
 }
 
-// y may be x (in place)
-__global__ void activation_kernel(const float *x, float *y, size_t count, int act)
+// y may be x (in place); vec_ok: both 16-byte aligned
+__global__ void activation_kernel(const float *x, float *y, size_t count, int act, int vec_ok)
 {
     pdl_wait();
-    for(size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x)
-        y[i] = apply_act(x[i], act);
+    const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+    size_t i = tid;
+    if(vec_ok) {
+        const size_t n4 = count / 4;
+        for(size_t j = tid; j < n4; j += step) {
+            float4 v = reinterpret_cast<const float4 *>(x)[j];
+            v.x = apply_act(v.x, act);
+            v.y = apply_act(v.y, act);
+            v.z = apply_act(v.z, act);
+            v.w = apply_act(v.w, act);
+            reinterpret_cast<float4 *>(y)[j] = v;
+        }
+        i = n4 * 4 + tid;
+    }
+    for(; i < count; i += step) y[i] = apply_act(x[i], act);
 }
 
 // one CTA per (row, inner) slice; classes strided by `inner`
@@ -263,17 +276,56 @@ __global__ void softmax_kernel(const float *x, float *y, int classes, int inner,
     }
 }
 
-__global__ void batchnorm_inference_kernel(const float *x, float *y, size_t count, int features, int plane,
-                                           float eps, const float *__restrict__ mean, const float *__restrict__ var,
-                                           const float *__restrict__ gamma, const float *__restrict__ beta)
+// y = a[f] * x + b[f], f the feature of the element's plane.  Memory-bound, if the index arithmetic lets it: a 64-bit division and a
+// remainder, a square root and a division for every element took three times as long as the bytes.  A thread takes four
+// consecutive elements (16-byte accesses, vec_ok: aligned) and works out plane and coefficients once for them when they lie in
+// one plane (plane % 4 == 0), with 32-bit divisions (Index = unsigned) when the tensor has fewer than 2^32 elements.
+// y may be x (in place).
+template<typename Index>
+__global__ void __launch_bounds__(256) batchnorm_inference_kernel(const float *x, float *y, Index count, Index features, Index plane, float eps,
+                                                                  const float *__restrict__ mean, const float *__restrict__ var,
+                                                                  const float *__restrict__ gamma, const float *__restrict__ beta, int vec_ok)
 {
     pdl_wait();
-    for(size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x) {
-        const int f = int((i / plane) % features);
-        float a = 1.0f / sqrtf(var[f] + eps);
-        float b = -mean[f] * a;
-        if(gamma && beta) { a *= gamma[f]; b = gamma[f] * b + beta[f]; }
-        y[i] = a * x[i] + b;
+    auto coefficients = [&](Index i) {
+        const Index f = (i / plane) % features;
+        float a = 1.0f / sqrtf(__ldg(var + f) + eps);
+        float b = -__ldg(mean + f) * a;
+        if(gamma && beta) {
+            const float g = __ldg(gamma + f);
+            a *= g;
+            b = g * b + __ldg(beta + f);
+        }
+        return make_float2(a, b);
+    };
+    const Index tid = blockIdx.x * Index(blockDim.x) + threadIdx.x, step = Index(gridDim.x) * blockDim.x, n4 = count / 4;
+    const bool one_plane = plane % 4 == 0;
+    for(Index j = tid; j < n4; j += step) {
+        const Index i = 4 * j;
+        float v[4];
+        if(vec_ok) {
+            const float4 t = reinterpret_cast<const float4 *>(x)[j];
+            v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+        }
+        else {
+            #pragma unroll
+            for(int k = 0; k < 4; k++) v[k] = x[i + k];
+        }
+        float2 c = coefficients(i);
+        #pragma unroll
+        for(int k = 0; k < 4; k++) {
+            if(k > 0 && !one_plane) c = coefficients(i + k);
+            v[k] = c.x * v[k] + c.y;
+        }
+        if(vec_ok) reinterpret_cast<float4 *>(y)[j] = make_float4(v[0], v[1], v[2], v[3]);
+        else {
+            #pragma unroll
+            for(int k = 0; k < 4; k++) y[i + k] = v[k];
+        }
+    }
+    for(Index i = 4 * n4 + tid; i < count; i += step) {
+        const float2 c = coefficients(i);
+        y[i] = c.x * x[i] + c.y;
     }
 }
 
@@ -393,8 +445,10 @@ dlp_status dlp_activation_fwd(const float *x, float *y, size_t count, int activa
 {
     DLP_REQUIRE(x && y, "null tensor");
     if(count == 0) return DLP_OK;
-    DLP_LAUNCH_PDL(launch_pdl(one_wave(grid_for(count, 256), 256), activation_kernel, grid_for(count, 256), 256, 0, (cudaStream_t)stream, x,
-                   y, count, activation), "activation_kernel");
+    const int vec_ok = (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) % 16 == 0;
+    const int grid = grid_for(count / (vec_ok ? 4 : 1) + 1, 256);
+    DLP_LAUNCH_PDL(launch_pdl(one_wave(grid, 256), activation_kernel, grid, 256, 0, (cudaStream_t)stream, x, y, count, activation, vec_ok),
+                   "activation_kernel");
     return DLP_OK;
 }
 
@@ -416,8 +470,17 @@ dlp_status dlp_batchnorm_inference_fwd(const float *x, float *y, int batch, int 
     DLP_REQUIRE(features > 0 && plane > 0, "bad batch-norm shape");
     const size_t count = size_t(batch) * features * plane;
     if(count == 0) return DLP_OK;
-    DLP_LAUNCH_PDL(launch_pdl(one_wave(grid_for(count, 256), 256), batchnorm_inference_kernel, grid_for(count, 256), 256, 0,
-                   (cudaStream_t)stream, x, y, count, features, plane, eps, mean, var, gamma, beta), "batchnorm_inference_kernel");
+    const int vec_ok = (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) % 16 == 0;
+    const int grid = grid_for(count / 4 + 1, 256);
+    // 2^31: the loops' indexes step beyond the end by a grid's worth of elements
+    if(count < (size_t(1) << 31))
+        DLP_LAUNCH_PDL(launch_pdl(one_wave(grid, 256), batchnorm_inference_kernel<unsigned>, grid, 256, 0, (cudaStream_t)stream, x, y,
+                                  unsigned(count), unsigned(features), unsigned(plane), eps, mean, var, gamma, beta, vec_ok),
+                       "batchnorm_inference_kernel");
+    else
+        DLP_LAUNCH_PDL(launch_pdl(one_wave(grid, 256), batchnorm_inference_kernel<size_t>, grid, 256, 0, (cudaStream_t)stream, x, y, count,
+                                  size_t(features), size_t(plane), eps, mean, var, gamma, beta, vec_ok),
+                       "batchnorm_inference_kernel");
     return DLP_OK;
 }
 
