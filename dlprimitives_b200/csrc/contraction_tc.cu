@@ -773,21 +773,23 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
 // A thread packs one 16-byte chunk (four consecutive k of one column): the swizzle permutes whole chunks, so the chunk is one
 // 16-byte store per tile.  n_major: consecutive threads take consecutive columns (sources whose columns are contiguous),
 // otherwise consecutive chunks along k (sources whose k is contiguous, read 16 bytes at a time when aligned).
+// Index: unsigned when the chunks of a matrix are fewer than 2^31 (a 64-bit division per chunk cost more than its bytes).
+template<typename Index>
 __global__ void prepack_kernel(const float *__restrict__ b, long long col_stride, long long k_stride, int cols, int k,
                                int n_pad, int k_pad, int bn, int taps, float *__restrict__ packed, long long b_batch_stride, int n_major,
                                int row_kw)
 {
     pdl_wait();
     const int chunks = k_pad / 4;
-    const long long total = (long long)n_pad * chunks;
+    const Index total = Index(n_pad) * Index(chunks);
     b += blockIdx.y * b_batch_stride;           // a batch of matrices: blockIdx.y picks one, packed one after the other
     packed += blockIdx.y * (2ll * n_pad * k_pad);
     const int kblocks = k_pad / BK;
     const bool vec = !n_major && taps == 0 && row_kw == 0 && k_stride == 1 && (col_stride & 3) == 0 && (reinterpret_cast<uintptr_t>(b) & 15) == 0;
-    for(long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
+    for(Index idx = blockIdx.x * Index(blockDim.x) + threadIdx.x; idx < total; idx += Index(gridDim.x) * blockDim.x) {
         int n, c;
-        if(n_major) { c = int(idx / n_pad); n = int(idx - (long long)c * n_pad); }
-        else { n = int(idx / chunks); c = int(idx - (long long)n * chunks); }
+        if(n_major) { c = int(idx / Index(n_pad)); n = int(idx - Index(c) * Index(n_pad)); }
+        else { n = int(idx / Index(chunks)); c = int(idx - Index(n) * Index(chunks)); }
         const int kk = c * 4, kb = kk / BK, i = kk % BK;
         float v[4] = { 0.0f, 0.0f, 0.0f, 0.0f };
         if(n < cols) {
@@ -829,19 +831,45 @@ __global__ void prepack_kernel(const float *__restrict__ b, long long col_stride
 }
 
 // Second step of a split-K contraction: add the partial results in a fixed order (so the sum does not
-// depend on timing) and apply the epilogue.  Partials are column-major [part][col][rows_pad].
-__global__ void split_finish_kernel(const Contraction p, const float *__restrict__ partial, int splits, long long split_stride, long long rows_pad)
+// depend on timing) and apply the epilogue.  Partials are column-major [part][col][rows_pad], rows_pad a multiple of 128.
+// A thread takes four consecutive rows of a column (16-byte loads) and asks for the partials of up to eight parts at a time:
+// one element at a time, part after part, the trips to L2 added up (sixteen parts of a 1 x 1000 result took longer than the
+// products; two parts of a 3136 x 1024 one moved 1.4 TB/s).  Index arithmetic in 32 bits when the quads are fewer than 2^31.
+template<typename Index>
+__global__ void __launch_bounds__(256) split_finish_kernel(const Contraction p, const float *__restrict__ partial, int splits,
+                                                           long long split_stride, long long rows_pad)
 {
     pdl_wait();
-    const long long total = p.rows * p.cols;
-    for(long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
-        const int col = int(idx / p.rows);
-        const long long row = idx - (long long)col * p.rows;
+    const Index quads = Index((p.rows + 3) / 4), total = quads * Index(p.cols);
+    for(Index idx = blockIdx.x * Index(blockDim.x) + threadIdx.x; idx < total; idx += Index(gridDim.x) * blockDim.x) {
+        const int col = int(idx / quads);
+        const long long row = 4 * (long long)(idx - Index(col) * quads);
         const float *src = partial + (long long)col * rows_pad + row;
-        float acc = __ldg(src);
-        for(int s = 1; s < splits; s++) acc += __ldg(src + s * split_stride);
-        const RowInfo r = make_row(p, row);
-        p.y[out_index(p, r, col)] = finish_output(p, r, row, col, acc);
+        float4 acc = __ldg(reinterpret_cast<const float4 *>(src));
+        #pragma unroll 1
+        for(int s = 1; s < splits; s += 8) {
+            float4 v[8];
+            #pragma unroll
+            for(int j = 0; j < 8; j++)
+                if(s + j < splits) v[j] = __ldg(reinterpret_cast<const float4 *>(src + (s + j) * split_stride));
+            #pragma unroll
+            for(int j = 0; j < 8; j++)
+                if(s + j < splits) { acc.x += v[j].x; acc.y += v[j].y; acc.z += v[j].z; acc.w += v[j].w; }
+        }
+        const float a[4] = { acc.x, acc.y, acc.z, acc.w };
+        RowInfo r = make_row(p, row);
+        // the four rows follow each other in y when they are pixels of one image, or y is column-major
+        const bool together = p.out_mode == OUT_COL_MAJOR || (p.out_mode == OUT_NCHW && p.plane % 4 == 0);
+        const long long step = p.out_mode == OUT_ROW_MAJOR ? p.ldc : 1;
+        #pragma unroll
+        for(int j = 0; j < 4; j++) {
+            if(row + j >= p.rows) break;
+            if(j > 0) {
+                if(together || p.out_mode == OUT_ROW_MAJOR) r.out += step;
+                else r = make_row(p, row + j);
+            }
+            p.y[out_index(p, r, col)] = finish_output(p, r, row + j, col, a[j]);
+        }
     }
 }
 
@@ -865,30 +893,32 @@ dlp_status tc_prepack(const TcPacked &L, const float *b, long long b_col_stride,
     const int threads = 256;
     const int blocks = int(std::min<long long>(ceil_div<long long>(total, threads), 8 * sm_count()));
     if(batch < 1 || batch > 65535) return fail(DLP_INVALID_ARGUMENT, "a batched product takes 1 to 65535 matrices");
-    DLP_LAUNCH_PDL(launch_pdl(one_wave((long long)blocks * batch, threads), tc::prepack_kernel, dim3(blocks, batch), threads, 0, stream, b,
-                   b_col_stride, b_k_stride, cols, k, L.n_pad, L.k_pad, L.bn, taps, packed, b_batch_stride,
-                   b_col_stride == 1 && b_k_stride != 1 ? 1 : 0, row_kw), "prepack_kernel");
+    const auto pack = total < (1ll << 31) ? tc::prepack_kernel<unsigned> : tc::prepack_kernel<long long>;
+    DLP_LAUNCH_PDL(launch_pdl(one_wave((long long)blocks * batch, threads), pack, dim3(blocks, batch), threads, 0, stream, b, b_col_stride, b_k_stride,
+                              cols, k, L.n_pad, L.k_pad, L.bn, taps, packed, b_batch_stride, b_col_stride == 1 && b_k_stride != 1 ? 1 : 0, row_kw),
+                   "prepack_kernel");
     return DLP_OK;
 }
 
 namespace {
-// How many equal parts to cut K into.  Time is counted in k-block periods (about 0.6 us): a CTA works through
+// How many equal parts to cut K into.  Time is counted in k-block periods (about 0.5 us): a CTA works through
 // ceil(items / SMs) work items of (k-blocks per part + a fixed cost for pipeline fill and epilogue) each,
 // and a split run pays for the finishing kernel.  K is cut only when that model gains a tenth or more.
-// The two constants are fitted to timings of batch-32 layer shapes with forced splits (52 to 196 tiles of 16 to 144
-// k-blocks): 7 periods per work item, 20 for the second launch and its pass over the partial sums.
+// The constants are fitted to timings of batch-1 and batch-16 layer shapes with forced splits: 7 periods per work item; 3 for
+// the second launch, which starts under the first (3x3 512 -> 512 on 7x7, one image: 144 k-blocks 82 us, two parts 47, four 30,
+// eight 21), and its pass over the partial sums, written and read, at 2 MB a period.
 int choose_splits(long long rows, const TcPacked &L)
 {
     const long long tiles = ceil_div<long long>(rows, tc::BM) * (L.n_pad / L.bn);
     const int kb = L.k_pad / tc::BK, sms = sm_count();
     if(tiles <= 0 || tiles > 4 * sms || kb < 8) return 1;
-    const double item_fixed = 7.0, finish = 20.0;
+    const double item_fixed = 7.0, finish = 3.0, per_part = double(rows) * L.n_pad * sizeof(float) / 2e6;
     const double uncut = double(ceil_div<long long>(tiles, sms)) * (kb + item_fixed);
     int best = 1;
     double best_cost = 0.9 * uncut;
     for(int s = 2; s <= 32 && kb / s >= 4; s++) {
         if(kb % s != 0) continue;
-        const double cost = double(ceil_div<long long>(tiles * s, sms)) * (kb / s + item_fixed) + finish;
+        const double cost = double(ceil_div<long long>(tiles * s, sms)) * (kb / s + item_fixed) + finish + per_part * (2 * s + 1);
         if(cost < best_cost) { best = s; best_cost = cost; }
     }
     return best;
@@ -1007,10 +1037,11 @@ dlp_status launch_contraction_tc(const Contraction &p, const TcPacked &L, const 
     default: return fail(DLP_INVALID_ARGUMENT, "unsupported column tile");
     }
     if(st != DLP_OK || splits == 1) return st;
-    const long long total = p.rows * p.cols;
-    const int blocks = int(std::min<long long>(ceil_div<long long>(total, 256), 16 * sm_count()));
-    DLP_LAUNCH_PDL(launch_pdl(one_wave(blocks, 256), tc::split_finish_kernel, blocks, 256, 0, stream, p,
-                   static_cast<const float *>(scratch), splits, split_stride, rows_pad), "split_finish_kernel");
+    const long long quads = (p.rows + 3) / 4 * p.cols;
+    const int blocks = int(std::min<long long>(ceil_div<long long>(quads, 256), 16 * sm_count()));
+    const auto finish = quads < (1ll << 31) ? tc::split_finish_kernel<unsigned> : tc::split_finish_kernel<long long>;
+    DLP_LAUNCH_PDL(launch_pdl(one_wave(blocks, 256), finish, blocks, 256, 0, stream, p, static_cast<const float *>(scratch), splits, split_stride,
+                              rows_pad), "split_finish_kernel");
     return DLP_OK;
 }
 
