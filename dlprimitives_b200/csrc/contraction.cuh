@@ -75,6 +75,10 @@ struct Contraction {
     int post_act;
 };
 
+// Quotient of work item numbers, in 32 bits: a tile is at least 128 rows by a column, so 2^31 items would be outputs of more than
+// a terabyte.  (A 64-bit division takes hundreds of cycles, and a block did several before its first load: 2000 cycles in all.)
+__device__ __forceinline__ long long div32(long long a, long long b) { return (long long)(unsigned(a) / unsigned(b)); }
+
 // Row (pixel) coordinates shared by the loaders.
 struct RowInfo {
     long long base;  // element offset of the row's first tap (may be "negative" through padding)

@@ -192,7 +192,8 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *(volatile uint32_t *)&sh->tmem_base;
-    pdl_wait();          // everything up to here ran under the kernel before; from here on global memory is read
+    // (Each role waits for the kernel before, pdl_wait(), where it first touches global memory: barriers, tensor memory and the
+    // arithmetic of the first work item are done under that kernel.)
 
     // ---- epilogue pieces shared by the accumulate warps and, for a CTA's last work item, the loader warps
     // identity / relu / relu6 are a clamp; with no per-row bias and no beta the whole epilogue is
@@ -204,7 +205,7 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
     constexpr int G = BN >= 32 ? 32 : 16;
     constexpr int GROUPS = BN / G;
     const int chunks_per_tile = (kblocks + CHUNK_KB - 1) / CHUNK_KB;
-    const long long my_items = blockIdx.x < num_tiles ? (num_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+    const long long my_items = blockIdx.x < num_tiles ? div32(num_tiles - blockIdx.x + gridDim.x - 1, gridDim.x) : 0;
     // The epilogue of a CTA's last work item has nothing to hide behind.  When that tile is a whole one on the lean path,
     // the loader warps (idle by then) take column groups of its last chunk: group 0 stays with the accumulate warps, 1 and 3
     // go to the first loader group, 2 to the second.  Every side derives the decision from the same CTA-wide values.
@@ -214,7 +215,7 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
         long long t;
         int part_unused;
         decode_item(last_item, splits, t, part_unused);
-        tail_help = int(t % n_tiles) * BN + BN <= p.cols;
+        tail_help = int(t - div32(t, n_tiles) * n_tiles) * BN + BN <= p.cols;
     }
     auto tail_owner = [](int g) { return g == 0 ? 0 : (g == 2 ? 2 : 1); };   // 0: accumulate warps, 1 / 2: loader groups
     struct EpiItem {
@@ -229,8 +230,9 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
         EpiItem e;
         long long tile;
         decode_item(item, splits, tile, e.part);
-        e.n0 = int(tile % n_tiles) * BN;
-        e.row = (tile / n_tiles) * BM + row_in_tile;
+        const long long row_tile = div32(tile, n_tiles);
+        e.n0 = int(tile - row_tile * n_tiles) * BN;
+        e.row = row_tile * BM + row_in_tile;
         e.r = make_row(p, e.row, a_off, y_off);
         e.col_stride = p.out_mode == OUT_NCHW ? (long long)p.plane : (p.out_mode == OUT_COL_MAJOR ? p.ldc : 1ll);
         e.fast = epi_fast && e.r.valid && e.n0 + BN <= p.cols && !TC_DIAG(DIAG_NO_STORES);
@@ -313,7 +315,8 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
                 long long tile;
                 int part;
                 decode_item(item, splits, tile, part);
-                const float *src = packed + ((long long)(tile % n_tiles) * splits + part) * kblocks * (B_STAGE_BYTES / 4);
+                const float *src = packed + ((tile - div32(tile, n_tiles) * n_tiles) * splits + part) * kblocks * (B_STAGE_BYTES / 4);
+                if(it == 0) pdl_wait();
                 for(int kb = 0; kb < kblocks; kb++, it++) {
                     const int s = it % STAGES;
                     if(!mbar_wait(&sh->empty[s >> 1], ((it / STAGES) & 1) ^ 1, &sh->abort_flag, status, ST_TMA_EMPTY)) { live = false; break; }
@@ -342,7 +345,7 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
         const uint32_t acc_empty0 = smem_u32(&sh->acc_empty[0]), empty0 = smem_u32(&sh->empty[0]), acc_full0 = smem_u32(&sh->acc_full[0]);
         // the barrier array this lane watches (8 bytes per entry): even lanes the A columns, odd lanes the B tiles
         const uint32_t watch_base = smem_u32(lane & 1 ? &sh->full_b[0] : &sh->full_a[0]);
-        const long long my_tiles = blockIdx.x < num_tiles ? (num_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+        const long long my_tiles = blockIdx.x < num_tiles ? div32(num_tiles - blockIdx.x + gridDim.x - 1, gridDim.x) : 0;
         const uint32_t total = uint32_t(my_tiles * kblocks);
         uint32_t chunk = 0, s = 0, s_phase = 0;           // partial accumulators so far; ring position and parity
         int kb = 0, in_chunk = 0;
@@ -436,6 +439,7 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
         // Worth it (measured) when a tile has 3 to 8 k-blocks: with fewer the tiles are too short to stay a tile
         // ahead, with more the MMAs hide the epilogue anyway.
         if(p.residual != nullptr && !short_k && kblocks <= CHUNK_KB) {
+            pdl_wait();
             // item index i of this CTA is prefetched once the accumulate warps have started on item i - 1
             // (a counter they publish); when this warp has fallen behind it skips to where they are
             uint32_t i = 0;
@@ -450,8 +454,9 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
                 long long tile;
                 int part;
                 decode_item(item, splits, tile, part);
-                const int n0 = int(tile % n_tiles) * BN;
-                const long long row0 = (tile / n_tiles) * BM;
+                const long long row_tile = div32(tile, n_tiles);
+                const int n0 = int(tile - row_tile * n_tiles) * BN;
+                const long long row0 = row_tile * BM;
                 // every 16th row of the tile (64 bytes apart in a channel plane), and its last row: touches every line
                 #pragma unroll 1
                 for(int j = 0; j <= BM / 16; j++) {
@@ -474,6 +479,7 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
         float *my_sums = sums + row_in_tile;                // element (col) at my_sums[col * BM]: conflict-free
         uint32_t chunk = 0, items_begun = 0;
         bool live = true;
+        pdl_wait();
         for(long long item = blockIdx.x; item < num_tiles && live; item += gridDim.x) {
             const EpiItem e = epi_item(item, row_in_tile);
             const RowInfo &r = e.r;
@@ -573,7 +579,7 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
             if(c.tile != loaded_tile) {
                 loaded_tile = c.tile;
                 decode_item(c.tile, splits, loaded_row_tile, loaded_part);
-                r = make_row(p, (loaded_row_tile / n_tiles) * BM + row_in_tile, a_off, y_off);
+                r = make_row(p, div32(loaded_row_tile, n_tiles) * BM + row_in_tile, a_off, y_off);
                 if(TC_DIAG(DIAG_NO_A_LOADS)) r.valid = false;
                 row_mask = col_mask = 0;
                 if((MODE == A_GATHER || MODE == A_ROWTAPS) && r.valid) {
@@ -705,6 +711,7 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
         advance(nxt, group);
         cur = nxt;
         bool have_cur = false;
+        pdl_wait();
         #pragma unroll 1
         for(;;) {
             const bool more = nxt.tile < num_tiles;
@@ -722,10 +729,10 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
         // ---- the last chunk of the CTA's last work item: this loader group's share of the epilogue
         if(tail_help && !*(volatile int *)&sh->abort_flag) {
             const uint32_t last_chunk = uint32_t(my_items * chunks_per_tile - 1), buf = last_chunk & 1;
+            const EpiItem e = epi_item(last_item, row_in_tile);
             if(warp_wait(&sh->sums_ready, 0, &sh->abort_flag, status, ST_EPI_ACC, lane) &&
                warp_wait(&sh->acc_full[buf], (last_chunk >> 1) & 1, &sh->abort_flag, status, ST_EPI_ACC, lane)) {
                 tc_fence_after();
-                const EpiItem e = epi_item(last_item, row_in_tile);
                 const uint32_t taddr = tmem_base + (uint32_t(quad * 32) << 16) + buf * BN;
                 #pragma unroll 1
                 for(int g = 1; g < GROUPS; g++)
@@ -998,6 +1005,8 @@ dlp_status launch_contraction_tc(const Contraction &p, const TcPacked &L, const 
     if(p.rows <= 0 || p.cols <= 0 || batch.count <= 0) return DLP_OK;
     if(reinterpret_cast<uintptr_t>(packed) % 16 != 0) return fail(DLP_INVALID_ARGUMENT, "packed weights must be 16-byte aligned");
     if(batch.count > 65535) return fail(DLP_INVALID_ARGUMENT, "a batched product takes at most 65535 matrices");
+    if(ceil_div<long long>(p.rows, tc::BM) * ceil_div(p.cols, L.bn) * batch.count >= (1ll << 31))
+        return fail(DLP_INVALID_ARGUMENT, "more than 2^31 output tiles");
     int splits = batch.count > 1 ? 1 : choose_splits(p.rows, L);      // the matrices of a batch fill the GPU between them
     if(splits == 1 && batch.count == 1 && pointwise_tc_eligible(p, L)) return launch_pointwise_tc(p, L, packed, stream);
     // (environment variable DLP_TC_NO_STAGED: keep such problems on this file's kernel, for A/B timing and profiling)

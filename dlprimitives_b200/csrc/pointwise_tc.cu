@@ -93,9 +93,9 @@ struct Item {
 __device__ __forceinline__ Item decode(long long item, const Params &q)
 {
     Item w;
-    const long long m_tile = item / q.n_tiles;
+    const long long m_tile = div32(item, q.n_tiles);
     w.n_tile = int(item - m_tile * q.n_tiles);
-    w.b = int(m_tile / q.tiles_per_image);
+    w.b = int(div32(m_tile, q.tiles_per_image));
     w.pix0 = int(m_tile - (long long)w.b * q.tiles_per_image) * BM;
     return w;
 }
@@ -144,7 +144,7 @@ pointwise_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
     const int kblocks = q.kblocks;
     // a warp with nothing else to do issues MMAs too: the B warp once resident weights are in, else the residual warp of a launch without residual
     const int second_issuer = q.resident ? WARP_B : (q.has_res ? -1 : WARP_RES);
-    const long long my_items = blockIdx.x < q.num_items ? (q.num_items - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+    const long long my_items = blockIdx.x < q.num_items ? div32(q.num_items - blockIdx.x + gridDim.x - 1, gridDim.x) : 0;
 
     if(threadIdx.x == 0) {
         for(int s = 0; s < MAX_S_STAGES; s++) { mbar_init(&sh->sa_full[s], 1); mbar_init(&sh->sa_empty[s], 4); }
@@ -164,11 +164,12 @@ pointwise_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *(volatile uint32_t *)&sh->tmem_base;
-    pdl_wait();          // everything up to here ran under the kernel before; from here on global memory is read
+    // (each role waits for the kernel before, pdl_wait(), where it first touches global memory)
 
     if(warp == WARP_B) {
         // ------------------------------------------------------------------ B copies
         if(lane == 0) {
+            pdl_wait();
             if(q.resident) {
                 // the CTA's column tile never changes: its k-blocks go to stages 0 .. kblocks-1 once
                 if(my_items > 0) {
@@ -203,6 +204,7 @@ pointwise_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
     if(warp == WARP_A) {
         // ------------------------------------------------------------------ A copies
         if(lane == 0) {
+            pdl_wait();
             uint32_t it = 0;
             bool live = true;
             for(long long item = blockIdx.x; item < q.num_items && live; item += gridDim.x) {
@@ -220,6 +222,7 @@ pointwise_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
     else if(warp == WARP_RES && q.has_res) {
         // ------------------------------------------------------------------ residual copies
         if(lane == 0) {
+            pdl_wait();
             uint32_t j = 0;
             bool live = true;
             for(long long item = blockIdx.x; item < q.num_items && live; item += gridDim.x) {
@@ -329,6 +332,7 @@ pointwise_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
         const bool release_at_once = q.has_res || E_BUFS < 2 * SETS;
         bool live = true;
         long long i = 0;
+        pdl_wait();
         for(long long item = blockIdx.x; item < q.num_items && live; item += gridDim.x, i++) {
             const Item w = decode(item, q);
             const uint32_t buf = uint32_t(i) & 1;

@@ -95,9 +95,9 @@ struct Item {
 __device__ __forceinline__ Item decode(long long item, const Params &q)
 {
     Item w;
-    const long long m_tile = item / q.n_tiles;
+    const long long m_tile = div32(item, q.n_tiles);
     w.n_tile = int(item - m_tile * q.n_tiles);
-    w.b = int(m_tile / q.tiles_per_image);
+    w.b = int(div32(m_tile, q.tiles_per_image));
     w.t = int(m_tile - (long long)w.b * q.tiles_per_image);
     return w;
 }
@@ -151,7 +151,7 @@ staged_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kblocks = q.kblocks;
-    const long long my_items = blockIdx.x < q.num_items ? (q.num_items - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+    const long long my_items = blockIdx.x < q.num_items ? div32(q.num_items - blockIdx.x + gridDim.x - 1, gridDim.x) : 0;
 
     if(threadIdx.x == 0) {
         for(int s = 0; s < MAX_S_STAGES; s++) { mbar_init(&sh->sa_full[s], 1); mbar_init(&sh->sa_empty[s], 8); }
@@ -187,11 +187,12 @@ staged_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *(volatile uint32_t *)&sh->tmem_base;
-    pdl_wait();          // everything up to here ran under the kernel before; from here on global memory is read
+    // (each role waits for the kernel before, pdl_wait(), where it first touches global memory)
 
     if(warp == WARP_A) {
         // ------------------------------------------------------------------ patch copies
         if(lane == 0) {
+            pdl_wait();
             uint32_t pi = 0;
             bool live = true;
             for(long long item = blockIdx.x; item < q.num_items && live; item += gridDim.x) {
@@ -210,6 +211,7 @@ staged_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
     else if(warp == WARP_B) {
         // ------------------------------------------------------------------ B copies
         if(lane == 0) {
+            pdl_wait();
             if(q.resident) {
                 // the CTA's column tile never changes: its k-blocks go to stages 0 .. kblocks-1 once
                 if(my_items > 0) {
@@ -328,6 +330,7 @@ staged_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
         uint32_t chunk = 0;
         bool live = true;
         long long i = 0;
+        pdl_wait();
         for(long long item = blockIdx.x; item < q.num_items && live; item += gridDim.x, i++) {
             const Item w = decode(item, q);
             // the bias of the set's 32 channels is asked for now: its trip to L2 is over long before the last chunk is in

@@ -122,7 +122,7 @@ __device__ __forceinline__ Item decode(long long item, const Params &q)
     Item w;
     w.z = 0;
     if(q.items_each != q.num_items) {
-        w.z = int(item / q.items_each);
+        w.z = int(div32(item, q.items_each));
         item -= w.z * q.items_each;
     }
     long long t = item;
@@ -131,7 +131,7 @@ __device__ __forceinline__ Item decode(long long item, const Params &q)
         t = unsigned(item) / unsigned(q.splits);           // few tiles whenever K is split
         w.part = int(unsigned(item) - unsigned(t) * unsigned(q.splits));
     }
-    const long long mt = t / q.n_tiles;
+    const long long mt = div32(t, q.n_tiles);
     w.n_tile = int(t - mt * q.n_tiles);
     w.m0 = mt * BM;
     return w;
@@ -174,7 +174,7 @@ stream_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const float *__re
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kblocks = q.kblocks, T = q.taps;
-    const long long my_items = blockIdx.x < q.num_items ? (q.num_items - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+    const long long my_items = blockIdx.x < q.num_items ? div32(q.num_items - blockIdx.x + gridDim.x - 1, gridDim.x) : 0;
 
     if(threadIdx.x == 0) {
         for(int s = 0; s < MAX_S_STAGES; s++) { mbar_init(&sh->sa_full[s], SRC == SRC_COPY ? 32 : 1); mbar_init(&sh->sa_empty[s], T == 1 ? 4 : 8); }
@@ -201,7 +201,7 @@ stream_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const float *__re
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *(volatile uint32_t *)&sh->tmem_base;
-    pdl_wait();          // everything up to here ran under the kernel before; from here on global memory is read
+    // (each role waits for the kernel before, pdl_wait(), where it first touches global memory)
 
     if(warp < WARP_ACC0) {
         regs_dec<REGS_ISSUE>();
@@ -217,7 +217,7 @@ stream_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const float *__re
                 const int c0 = w.part * slots;
                 int units = 1, my_x = 0, my_b = w.z;
                 if(!KMAJOR) {
-                    int u = 0, b = int(w.m0 / q.P), from = int(w.m0 - (long long)b * q.P), left = int(min((long long)BM, q.rows - w.m0));
+                    int u = 0, b = int(div32(w.m0, q.P)), from = int(w.m0 - (long long)b * q.P), left = int(min((long long)BM, q.rows - w.m0));
                     while(left > 0) {
                         const int n = min(left, q.P - from);
                         const int lo = max(from + q.dmin, 0) & ~3, hi = min(from + n + q.dmax, q.P);
@@ -230,6 +230,7 @@ stream_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const float *__re
                     }
                     units = u;
                 }
+                if(pi == 0) pdl_wait();
                 for(int c = 0; c < slots; c++, pi++) {
                     const int s = pi % S_STAGES;
                     if(!warp_wait(&sh->sa_empty[s], ((pi / S_STAGES) & 1) ^ 1, abort_flag, status, ST_A_EMPTY, lane)) { live = false; break; }
@@ -270,6 +271,7 @@ stream_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const float *__re
                     const Item w = decode(item, q);
                     const float *src = packed + (((long long)w.z * q.n_tiles + w.n_tile) * q.kblocks_all + (long long)w.part * kblocks) *
                                                 (B_STAGE_BYTES / 4);
+                    if(it == 0) pdl_wait();
                     for(int kb = 0; kb < kblocks; kb++, it++) {
                         const int s = it % B_STAGES;
                         if(!mbar_wait(&sh->empty_b[s], ((it / B_STAGES) & 1) ^ 1, abort_flag, status, ST_B_EMPTY)) { live = false; break; }
@@ -376,11 +378,12 @@ stream_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const float *__re
                 const Item w = decode(item, q);
                 const long long row = w.m0 + quad * 32 + lane;
                 const bool valid = row < q.rows;
-                const int b = valid ? int(row / q.P) : 0;
+                const int b = valid ? int(div32(row, q.P)) : 0;
                 const int pix = valid ? int(row - (long long)b * q.P) : 0;
                 const int col0 = w.n_tile * BN + set * COLS;
                 const long long off = w.z * q.y_batch_stride + w.part * q.y_split_stride + b * q.y_image_stride +
                                       pix * q.y_row_stride + col0 * q.y_col_stride;
+                if(item == blockIdx.x) pdl_wait();
                 // asked for now, used when the last chunk is in: the bias of the set's columns (handed round by shuffles), and the
                 // residual operand's lines into L2
                 float bias_g[COLS / 32];
@@ -483,9 +486,9 @@ stream_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const float *__re
             if(!KMAJOR && new_item) {
                 const Item w = decode(item, q);
                 const long long row = w.m0 + row_in_tile;
-                const int b0 = int(w.m0 / q.P), pix0 = int(w.m0 - (long long)b0 * q.P);
+                const int b0 = int(div32(w.m0, q.P)), pix0 = int(w.m0 - (long long)b0 * q.P);
                 valid = row < q.rows;
-                const int b = valid ? int(row / q.P) : b0;
+                const int b = valid ? int(div32(row, q.P)) : b0;
                 const int pix = valid ? int(row - (long long)b * q.P) : pix0;
                 const int lo0 = max(pix0 + q.dmin, 0) & ~3;
                 // units of the images before this one: the first from lo0 to its end, whole planes between
