@@ -778,8 +778,8 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
 // (see TcPacked): stage (column tile, k-block) = hi tile then lo tile, each bn rows of 32 floats with the
 // 16-byte chunks of a row permuted by the 128-byte swizzle (chunk ^ (row & 7)).
 // A thread packs one 16-byte chunk (four consecutive k of one column): the swizzle permutes whole chunks, so the chunk is one
-// 16-byte store per tile.  n_major: consecutive threads take consecutive columns (sources whose columns are contiguous),
-// otherwise consecutive chunks along k (sources whose k is contiguous, read 16 bytes at a time when aligned).
+// 16-byte store per tile.  n_major: a warp takes eight columns by four chunks (sources whose columns are contiguous),
+// otherwise consecutive threads take consecutive chunks along k (sources whose k is contiguous, read 16 bytes at a time when aligned).
 // Index: unsigned when the chunks of a matrix are fewer than 2^31 (a 64-bit division per chunk cost more than its bytes).
 template<typename Index>
 __global__ void prepack_kernel(const float *__restrict__ b, long long col_stride, long long k_stride, int cols, int k,
@@ -795,7 +795,14 @@ __global__ void prepack_kernel(const float *__restrict__ b, long long col_stride
     const bool vec = !n_major && taps == 0 && row_kw == 0 && k_stride == 1 && (col_stride & 3) == 0 && (reinterpret_cast<uintptr_t>(b) & 15) == 0;
     for(Index idx = blockIdx.x * Index(blockDim.x) + threadIdx.x; idx < total; idx += Index(gridDim.x) * blockDim.x) {
         int n, c;
-        if(n_major) { c = int(idx / Index(n_pad)); n = int(idx - Index(c) * Index(n_pad)); }
+        if(n_major) {
+            // a warp takes eight columns by four chunks: whole 32-byte sectors both where it reads (eight columns of a row of B) and where
+            // it writes (four chunks of a stage's row; one chunk in each of 32 rows would be half a sector each)
+            const Index g = idx >> 5;
+            const int lane = int(idx & 31), cg = int(g / Index(n_pad / 8)), ng = int(g - Index(cg) * Index(n_pad / 8));
+            n = ng * 8 + (lane & 7);
+            c = cg * 4 + (lane >> 3);
+        }
         else { n = int(idx / Index(chunks)); c = int(idx - Index(n) * Index(chunks)); }
         const int kk = c * 4, kb = kk / BK, i = kk % BK;
         float v[4] = { 0.0f, 0.0f, 0.0f, 0.0f };

@@ -52,16 +52,17 @@ struct Geometry {
     long long tiles, tiles_pad;
 };
 
-// one thread per (channel plane, tile): reads the 4x4 patch, writes the 16 transformed values (tiles contiguous across lanes)
+// one thread per (channel plane, tile): reads the 4x4 patch, writes the 16 transformed values (tiles contiguous across lanes).
+// Index: unsigned when (channel, tile) pairs fit 31 bits -- three 64-bit divisions per patch cost more than its bytes.
+template<typename Index>
 __global__ void wtc_input_kernel(const float *__restrict__ x, float *__restrict__ v, Geometry q)
 {
     pdl_wait();
-    const long long per_image = (long long)q.tiles_h * q.tiles_w;
-    const long long total = q.tiles * q.cin;
-    for(long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
-        const int c = int(idx / q.tiles);
-        const long long t = idx - (long long)c * q.tiles;
-        const int b = int(t / per_image), r = int(t - b * per_image);
+    const Index per_image = Index(q.tiles_h) * Index(q.tiles_w), tiles = Index(q.tiles), total = tiles * Index(q.cin);
+    for(Index idx = blockIdx.x * Index(blockDim.x) + threadIdx.x; idx < total; idx += Index(gridDim.x) * blockDim.x) {
+        const int c = int(idx / tiles);
+        const Index t = idx - Index(c) * tiles;
+        const int b = int(t / per_image), r = int(t - Index(b) * per_image);
         const int ty = r / q.tiles_w, tx = r - ty * q.tiles_w;
         const float *src = x + ((long long)b * q.cin + c) * q.h * q.w;
         float d[4][4];
@@ -102,15 +103,15 @@ struct OutArgs {
 };
 
 // one thread per (output channel plane, tile): reads the 16 products, writes the 2x2 outputs
+template<typename Index>
 __global__ void wtc_output_kernel(const float *__restrict__ mm, Geometry q, OutArgs a)
 {
     pdl_wait();
-    const long long per_image = (long long)q.tiles_h * q.tiles_w;
-    const long long total = q.tiles * q.cout;
-    for(long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
-        const int o = int(idx / q.tiles);
-        const long long t = idx - (long long)o * q.tiles;
-        const int b = int(t / per_image), r = int(t - b * per_image);
+    const Index per_image = Index(q.tiles_h) * Index(q.tiles_w), tiles = Index(q.tiles), total = tiles * Index(q.cout);
+    for(Index idx = blockIdx.x * Index(blockDim.x) + threadIdx.x; idx < total; idx += Index(gridDim.x) * blockDim.x) {
+        const int o = int(idx / tiles);
+        const Index t = idx - Index(o) * tiles;
+        const int b = int(t / per_image), r = int(t - Index(b) * per_image);
         const int ty = r / q.tiles_w, tx = r - ty * q.tiles_w;
         const float *src = mm + (long long)o * q.tiles_pad + t;
         const long long xi_stride = (long long)q.cout * q.tiles_pad;
@@ -189,7 +190,9 @@ dlp_status launch_winograd_tc(const float *x, const float *packed, const float *
     float *v = static_cast<float *>(ws);
     float *mm = v + 16ll * q.tiles_pad * cin;
     const int blocks = int(std::min<long long>(ceil_div<long long>(q.tiles * std::max(cin, cout), 256), 32ll * sm_count()));
-    DLP_LAUNCH_PDL(launch_pdl(one_wave(blocks, 256), wtc_input_kernel, blocks, 256, 0, stream, x, v, q), "wtc_input_kernel");
+    const bool narrow = q.tiles * std::max(cin, cout) < (1ll << 31);
+    const auto input = narrow ? wtc_input_kernel<unsigned> : wtc_input_kernel<long long>;
+    DLP_LAUNCH_PDL(launch_pdl(one_wave(blocks, 256), input, blocks, 256, 0, stream, x, v, q), "wtc_input_kernel");
 
     Contraction p;
     memset(&p, 0, sizeof(p));
@@ -213,7 +216,8 @@ dlp_status launch_winograd_tc(const float *x, const float *packed, const float *
 
     OutArgs a;
     a.bias = bias; a.residual = residual; a.y = y; a.act = act; a.post_act = post_act; a.factor = factor; a.residual_scale = residual_scale;
-    DLP_LAUNCH_PDL(launch_pdl(one_wave(blocks, 256), wtc_output_kernel, blocks, 256, 0, stream, mm, q, a), "wtc_output_kernel");
+    const auto output = narrow ? wtc_output_kernel<unsigned> : wtc_output_kernel<long long>;
+    DLP_LAUNCH_PDL(launch_pdl(one_wave(blocks, 256), output, blocks, 256, 0, stream, mm, q, a), "wtc_output_kernel");
     return DLP_OK;
 }
 
