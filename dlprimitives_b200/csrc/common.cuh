@@ -69,7 +69,8 @@ inline cudaError_t launch_pdl(bool early, void (*kernel)(P...), dim3 grid, dim3 
 
 // blocks of a plain kernel (threads each, little shared memory) that are all resident at once
 inline bool one_wave(long long blocks, int threads) { return blocks * threads <= (long long)sm_count() * 2048; }
-// work items of a persistent tensor-core kernel that are few enough for the set-up to matter
+// work items of a persistent tensor-core kernel that are few enough for the set-up to matter (3x3 64 -> 64 on 56x56 at batch 16, 448
+// items, with the packing of its weights before it: 43.0 us in stream order, 40.3 us started early)
 inline bool few_items(long long items) { return items <= 4ll * sm_count(); }
 
 // ---- device side ---------------------------------------------------------------------------------
