@@ -58,6 +58,7 @@ SYMBOLS = {
     "dlp_selftest_wait_expiry": (_i, [C.POINTER(C.c_int * 4), _vp]),
     "dlp_tf32_mma_rate": (_i, [C.POINTER(C.c_double), _vp]),
     "dlp_tf32_issue_probe": (_i, [C.c_int, C.c_int, C.POINTER(C.c_double), _vp]),
+    "dlp_pointwise_rings": (_i, [_i, _i, _i, _i, _ip, _ip]),
     "dlp_conv2d_output_shape": (_i, [C.POINTER(ConvDesc), _i, _i, _ip, _ip]),
     "dlp_conv2d_fwd_create": (_i, [C.POINTER(ConvDesc), C.POINTER(_vp)]),
     "dlp_conv2d_fwd_destroy": (None, [_vp]),

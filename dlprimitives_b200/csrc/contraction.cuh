@@ -165,6 +165,8 @@ dlp_status launch_contraction_tc(const Contraction &p, const TcPacked &L, const 
 // engines (pointwise_tc.cu).  launch_contraction_tc hands eligible problems over by itself.
 bool pointwise_tc_eligible(const Contraction &p, const TcPacked &L);
 dlp_status launch_pointwise_tc(const Contraction &p, const TcPacked &L, const float *packed, cudaStream_t stream);
+// depths of the shared-memory rings that its launches choose (dlp_pointwise_rings)
+dlp_status pointwise_rings(int bn, int kblocks, bool resident, bool has_res, int *a_slots, int *epilogue_buffers);
 
 // Convolutions with at most 64 output channels over rows of a multiple of four pixels (the 7x7 stem, 3x3 over 64 channels): the
 // input patch of a tile of whole output rows comes in by one tensor-map copy per channel block and every tap is gathered from

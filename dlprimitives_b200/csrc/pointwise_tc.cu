@@ -513,6 +513,35 @@ static dlp_status make_map(CUtensorMap &m, const float *base, int plane, int cha
     return DLP_OK;
 }
 
+constexpr int b_stage_bytes(int bn) { return 2 * bn * BK * 4; }
+
+// How shared memory is shared out: the weights first, the rest in 16 KB units between the A ring and the epilogue buffers.
+struct Rings { int b_bytes, s_stages, e_bufs; };
+static Rings rings(int bn, int kblocks, bool resident, bool has_res)
+{
+    Rings r;
+    r.b_bytes = (resident ? kblocks : T_STAGES) * b_stage_bytes(bn);
+    const int avail = (SMEM_LIMIT - SMEM_FIXED - r.b_bytes) / A_STAGE_BYTES;
+    if(avail <= 6 || (has_res && avail == 7)) {
+        // full weights region: a residual operand needs the buffers more than A needs depth
+        r.s_stages = has_res ? 2 : 4;
+        r.e_bufs = avail - r.s_stages;
+    }
+    else {
+        // An even number: the two converter groups take the k-blocks in turn, and with an odd one a group would meet ring entries
+        // whose last copy was the other group's.  A wait tells two successive copies of an entry apart only by one parity bit, so
+        // while that copy is still on its way the entry passes for filled: the group reads it too early, hands it back a
+        // second time, and from then on copies land in entries that are being read -- or after the block has left.
+        r.s_stages = (std::min(MAX_S_STAGES - 1, avail / 2) + 1) & ~1;
+        r.e_bufs = std::min(MAX_E_BUFS, avail - r.s_stages);
+    }
+    // The same for the buffers that a residual arrives in, which two sets of epilogue warps take in turn: with three of them a set
+    // could read one while the copy of the other set's group before it was still on its way (without a residual the wait is for the
+    // set's own stores, and any number serves).
+    if(has_res && bn > 32) r.e_bufs &= ~1;
+    return r;
+}
+
 template<int BN>
 static dlp_status launch_bn(const CUtensorMap &tx, const CUtensorMap &ty, const CUtensorMap &tr, const float *packed, const Params &q,
                             cudaStream_t stream)
@@ -533,24 +562,11 @@ static dlp_status launch_bn(const CUtensorMap &tx, const CUtensorMap &ty, const 
     if(!status) return fail(DLP_CUDA_ERROR, "cannot resolve the device status word");
     const int grid = int(std::min<long long>(q.num_items, sm_count()));
     Params r = q;
-    constexpr int b_stage_bytes = 2 * BN * BK * 4;
-    r.resident = q.kblocks * b_stage_bytes <= MAX_B_BYTES && grid % q.n_tiles == 0;
-    r.b_bytes = (r.resident ? q.kblocks : T_STAGES) * b_stage_bytes;
-    // the rest of shared memory in 16 KB units: split between the A ring and the epilogue buffers
-    const int avail = (SMEM_LIMIT - SMEM_FIXED - r.b_bytes) / A_STAGE_BYTES;
-    if(avail <= 6) {
-        // full weights region: a residual operand needs the buffers more than A needs depth
-        r.s_stages = q.has_res ? 2 : 4;
-        r.e_bufs = avail - r.s_stages;
-    }
-    else {
-        // An even number: the two converter groups take the k-blocks in turn, and with an odd one a group would meet ring entries
-        // whose last copy was the other group's.  A wait tells two successive copies of an entry apart only by one parity bit, so
-        // while that copy is still on its way the entry passes for filled: the group reads it too early, hands it back a
-        // second time, and from then on copies land in entries that are being read -- or after the block has left.
-        r.s_stages = (std::min(MAX_S_STAGES - 1, avail / 2) + 1) & ~1;
-        r.e_bufs = std::min(MAX_E_BUFS, avail - r.s_stages);
-    }
+    r.resident = q.kblocks * b_stage_bytes(BN) <= MAX_B_BYTES && grid % q.n_tiles == 0;
+    const Rings ring = rings(BN, q.kblocks, r.resident, q.has_res);
+    r.b_bytes = ring.b_bytes;
+    r.s_stages = ring.s_stages;
+    r.e_bufs = ring.e_bufs;
     const int smem_bytes = SMEM_FIXED + r.b_bytes + (r.s_stages + r.e_bufs) * A_STAGE_BYTES;
     DLP_LAUNCH_PDL(launch_pdl(few_items(q.num_items), pointwise_tf32x3_kernel<BN>, grid, NUM_THREADS, smem_bytes, stream, tx, ty, tr,
                    packed, r, status), "pointwise_tf32x3_kernel");
@@ -558,6 +574,17 @@ static dlp_status launch_bn(const CUtensorMap &tx, const CUtensorMap &ty, const 
 }
 
 } // namespace pw
+
+dlp_status pointwise_rings(int bn, int kblocks, bool resident, bool has_res, int *a_slots, int *epilogue_buffers)
+{
+    DLP_REQUIRE(a_slots && epilogue_buffers, "null result pointer");
+    DLP_REQUIRE((bn == 32 || bn == 64 || bn == 128) && kblocks >= 1 && kblocks <= 8, "column tile 32, 64 or 128, one to eight k-blocks");
+    DLP_REQUIRE(!resident || kblocks * pw::b_stage_bytes(bn) <= pw::MAX_B_BYTES, "weights too large to stay");
+    const pw::Rings r = pw::rings(bn, kblocks, resident, has_res);
+    *a_slots = r.s_stages;
+    *epilogue_buffers = r.e_bufs;
+    return DLP_OK;
+}
 
 bool pointwise_tc_eligible(const Contraction &p, const TcPacked &L)
 {

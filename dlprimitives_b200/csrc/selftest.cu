@@ -343,3 +343,8 @@ extern "C" dlp_status dlp_tf32_issue_probe(int scheme, int n, double *cycles_per
     default: return run_issue_probe<128, 3>(cycles_per_kblock, status, s);
     }
 }
+
+extern "C" dlp_status dlp_pointwise_rings(int bn, int kblocks, int resident, int residual, int *a_slots, int *epilogue_buffers)
+{
+    return pointwise_rings(bn, kblocks, resident != 0, residual != 0, a_slots, epilogue_buffers);
+}

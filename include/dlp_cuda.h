@@ -77,6 +77,11 @@ DLP_API dlp_status dlp_tf32_mma_rate(double *tflops, void *stream);
  * lane tests the same barriers (uniform instructions; the pointwise kernel's loop with resident weights); 3: two issuer warps taking pairs of
  * k-blocks in turn (what the contraction and staged kernels do).  Synchronises the stream. */
 DLP_API dlp_status dlp_tf32_issue_probe(int scheme, int n, double *cycles_per_kblock, void *stream);
+/* Depths of the shared-memory rings of the 1x1 kernel for a column tile of bn = 32, 64 or 128 channels and kblocks = 1..8 blocks of
+ * 32 input channels: slots of the input operand, and epilogue buffers (16 KB each).  resident: the weights stay in shared memory (at
+ * most 128 KB of them) instead of streaming through it.  A host-side rule, exposed so that the waits can be modelled with the depths that
+ * launches really use; needs no device. */
+DLP_API dlp_status dlp_pointwise_rings(int bn, int kblocks, int resident, int residual, int *a_slots, int *epilogue_buffers);
 
 /* ------------------------------------------------------------------------------------------------
  * Convolution forward.
