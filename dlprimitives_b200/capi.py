@@ -59,6 +59,7 @@ SYMBOLS = {
     "dlp_tf32_mma_rate": (_i, [C.POINTER(C.c_double), _vp]),
     "dlp_tf32_issue_probe": (_i, [C.c_int, C.c_int, C.POINTER(C.c_double), _vp]),
     "dlp_pointwise_rings": (_i, [_i, _i, _i, _i, _ip, _ip]),
+    "dlp_split_rule": (_i, [_ll, _i, _i, _vp, _sz, _ip, C.POINTER(_sz), C.POINTER(_sz)]),
     "dlp_conv2d_output_shape": (_i, [C.POINTER(ConvDesc), _i, _i, _ip, _ip]),
     "dlp_conv2d_fwd_create": (_i, [C.POINTER(ConvDesc), C.POINTER(_vp)]),
     "dlp_conv2d_fwd_destroy": (None, [_vp]),

@@ -1000,10 +1000,28 @@ dlp_status launch_bn(const Contraction &p, const TcPacked &L, const float *packe
 }
 } // namespace
 
+// The caller's scratch may start anywhere, the finishing kernel reads the partial sums 16 bytes at a time: they start at the scratch's
+// first 16-byte boundary, and SPLIT_ALIGN bytes are asked for beside them.
+static constexpr size_t SPLIT_ALIGN = 16;
+static size_t split_bytes(long long rows, const TcPacked &L, int parts)
+{
+    return size_t(parts) * size_t(round_up<long long>(rows, tc::BM)) * L.n_pad * sizeof(float);
+}
+
 size_t tc_split_scratch_bytes(long long rows, const TcPacked &L)
 {
     const int s = choose_splits(rows, L);
-    return s > 1 ? size_t(s) * size_t(ceil_div<long long>(rows, tc::BM) * tc::BM) * L.n_pad * sizeof(float) : 0;
+    return s > 1 ? split_bytes(rows, L, s) + SPLIT_ALIGN : 0;
+}
+
+int tc_split(long long rows, const TcPacked &L, void *scratch, size_t scratch_bytes, float **partial)
+{
+    *partial = nullptr;
+    const int s = choose_splits(rows, L);
+    const size_t skip = (SPLIT_ALIGN - reinterpret_cast<uintptr_t>(scratch) % SPLIT_ALIGN) % SPLIT_ALIGN;
+    if(s == 1 || scratch == nullptr || scratch_bytes < skip + split_bytes(rows, L, s)) return 1;
+    *partial = reinterpret_cast<float *>(static_cast<char *>(scratch) + skip);
+    return s;
 }
 
 dlp_status launch_contraction_tc(const Contraction &p, const TcPacked &L, const float *packed, cudaStream_t stream, void *scratch,
@@ -1021,11 +1039,12 @@ dlp_status launch_contraction_tc(const Contraction &p, const TcPacked &L, const 
     if(splits == 1 && batch.count == 1 && !no_staged && staged_tc_eligible(p, L)) return launch_staged_tc(p, L, packed, stream);
     const long long rows_pad = ceil_div<long long>(p.rows, tc::BM) * tc::BM;
     const long long split_stride = rows_pad * L.n_pad;
-    if(splits > 1 && (scratch == nullptr || scratch_bytes < size_t(splits) * split_stride * sizeof(float))) splits = 1;
+    float *partial = nullptr;
+    if(splits > 1) splits = tc_split(p.rows, L, scratch, scratch_bytes, &partial);
     Contraction q = p;
     if(splits > 1) {
         // the parts write raw partial sums to the scratch; the epilogue runs in the finishing kernel
-        q.y = static_cast<float *>(scratch);
+        q.y = partial;
         q.out_mode = OUT_COL_MAJOR;
         q.ldc = rows_pad;
         q.bias = nullptr;
@@ -1056,7 +1075,7 @@ dlp_status launch_contraction_tc(const Contraction &p, const TcPacked &L, const 
     const long long quads = (p.rows + 3) / 4 * p.cols;
     const int blocks = int(std::min<long long>(ceil_div<long long>(quads, 256), 16 * sm_count()));
     const auto finish = quads < (1ll << 31) ? tc::split_finish_kernel<unsigned> : tc::split_finish_kernel<long long>;
-    DLP_LAUNCH_PDL(launch_pdl(one_wave(blocks, 256), finish, blocks, 256, 0, stream, p, static_cast<const float *>(scratch), splits, split_stride,
+    DLP_LAUNCH_PDL(launch_pdl(one_wave(blocks, 256), finish, blocks, 256, 0, stream, p, partial, splits, split_stride,
                               rows_pad), "split_finish_kernel");
     return DLP_OK;
 }

@@ -348,3 +348,16 @@ extern "C" dlp_status dlp_pointwise_rings(int bn, int kblocks, int resident, int
 {
     return pointwise_rings(bn, kblocks, resident != 0, residual != 0, a_slots, epilogue_buffers);
 }
+
+extern "C" dlp_status dlp_split_rule(long long rows, int cols, int k, void *scratch, size_t scratch_bytes, int *parts, size_t *wanted_bytes,
+                                     size_t *offset)
+{
+    DLP_REQUIRE(parts && wanted_bytes && offset, "null result pointer");
+    DLP_REQUIRE(rows > 0 && cols > 0 && k > 0, "rows, columns and terms must be positive");
+    const TcPacked L = tc_packed_layout(cols, k);
+    float *partial = nullptr;
+    *parts = tc_split(rows, L, scratch, scratch_bytes, &partial);
+    *wanted_bytes = tc_split_scratch_bytes(rows, L);
+    *offset = partial ? size_t(reinterpret_cast<char *>(partial) - static_cast<char *>(scratch)) : 0;
+    return DLP_OK;
+}

@@ -82,6 +82,11 @@ DLP_API dlp_status dlp_tf32_issue_probe(int scheme, int n, double *cycles_per_kb
  * most 128 KB of them) instead of streaming through it.  A host-side rule, exposed so that the waits can be modelled with the depths that
  * launches really use; needs no device. */
 DLP_API dlp_status dlp_pointwise_rings(int bn, int kblocks, int resident, int residual, int *a_slots, int *epilogue_buffers);
+/* Into how many parts a product of rows x cols with k terms is cut when it is called with this scratch, the bytes of scratch that
+ * a plan for it asks for, and where in the scratch the partial sums go (offset in bytes).  A host-side rule; reads nothing through the
+ * pointer and needs no device. */
+DLP_API dlp_status dlp_split_rule(long long rows, int cols, int k, void *scratch, size_t scratch_bytes, int *parts, size_t *wanted_bytes,
+                                  size_t *offset);
 
 /* ------------------------------------------------------------------------------------------------
  * Convolution forward.
@@ -121,7 +126,7 @@ DLP_API const char *dlp_conv2d_fwd_kernel(const dlp_conv2d_plan *plan);
 /* Conv2DBase::workspace(): bytes of scratch enqueue needs for the planned batch: the packed weights, plus,
  * for problems with too few output tiles to fill the GPU, room for partial sums over parts of K (the
  * results are added in a fixed order, so they do not depend on timing).  enqueue_packed uses a workspace
- * only for the latter; a short or missing one just turns the split off. */
+ * only for the latter, at any address; a short or missing one just turns the split off. */
 DLP_API size_t dlp_conv2d_fwd_workspace(const dlp_conv2d_plan *plan);
 /* Bytes of the pre-packed form of the weights (0 when the kernel reads raw weights). */
 DLP_API size_t dlp_conv2d_fwd_packed_bytes(const dlp_conv2d_plan *plan);
@@ -204,7 +209,7 @@ DLP_API size_t dlp_ip_fwd_packed_bytes(const dlp_ip_plan *plan);
 DLP_API dlp_status dlp_ip_fwd_prepack(const dlp_ip_plan *plan, const float *w, void *packed, void *stream);
 DLP_API dlp_status dlp_ip_fwd_enqueue(const dlp_ip_plan *plan, const float *x, const float *w, const float *bias, float *y,
                                       void *ws, size_t ws_bytes, int batch, void *stream);
-/* ws: optional scratch (dlp_ip_fwd_workspace() bytes at most are used) that lets a small batch use the whole GPU. */
+/* ws: optional scratch (dlp_ip_fwd_workspace() bytes at most are used, at any address) that lets a small batch use the whole GPU. */
 DLP_API dlp_status dlp_ip_fwd_enqueue_packed(const dlp_ip_plan *plan, const float *x, const void *packed, const float *bias,
                                              float *y, void *ws, size_t ws_bytes, int batch, void *stream);
 
