@@ -564,7 +564,7 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
         r.valid = false; r.base = 0; r.iy0 = r.ix0 = 0; r.out = 0;
 
         const bool row_vec = MODE == A_STRIDED && p.plane == 0 && p.a_k_stride == 1 && (p.a_row_stride & 3) == 0 &&
-                             (reinterpret_cast<uintptr_t>(p.a) & 15) == 0;
+                             ((reinterpret_cast<uintptr_t>(p.a) + a_off * sizeof(float)) & 15) == 0;
         auto advance = [&](Cursor &c, int steps) {
             c.kb += steps;
             c.it += steps;

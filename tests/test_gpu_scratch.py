@@ -1,4 +1,5 @@
-"""Calls with packed weights whose scratch starts four bytes off a 16-byte boundary: the same parts, the same bits."""
+"""Buffers at addresses that 16-byte accesses cannot take: scratch that starts off a boundary (the same parts, the same bits), and
+matrices of a batch at strides that are no multiple of four."""
 import pytest
 import torch
 
@@ -23,3 +24,21 @@ def test_scratch_at_any_address(shift):
         plan.enqueue_packed(xt, packed, bias, y2, ws=ws[shift:])
         assert capi.device_status() == 0
         assert bool(y.isfinite().all()) and torch.equal(y, y2)
+
+
+@pytest.mark.parametrize("extra", [1, 2, 3, 4])
+def test_batched_matrices_at_any_stride(extra):
+    from dlprimitives_b200 import capi
+    g = torch.Generator(device=DEV).manual_seed(extra)
+    count, m, n, k = 3, 130, 96, 64
+    stride = m * k + extra
+    a = torch.randn(count * stride, device=DEV, generator=g)
+    b = torch.randn(count, n, k, device=DEV, generator=g)
+    plan = capi.Gemm(False, True, m, n, k)
+    c = torch.full((count, m, n), float("nan"), device=DEV)
+    ws = torch.empty(plan.batched_workspace(count), dtype=torch.uint8, device=DEV)
+    plan.batch_gemm(count, m, n, k, a, stride, k, b, n * k, k, c, m * n, n, ws=ws)
+    assert capi.device_status() == 0
+    rows = torch.stack([a[i * stride:i * stride + m * k].view(m, k) for i in range(count)])
+    want = torch.matmul(rows.double(), b.double().transpose(1, 2))
+    assert float((c.double() - want).norm() / want.norm()) < 5e-6       # as in test_gpu_stream.py
