@@ -903,6 +903,8 @@ TcPacked tc_packed_layout(int cols, int k)
 dlp_status tc_prepack(const TcPacked &L, const float *b, long long b_col_stride, long long b_k_stride, int cols, int k,
                       float *packed, int taps, cudaStream_t stream, int batch, long long b_batch_stride, int row_kw)
 {
+    // stored 16 bytes at a time
+    if(reinterpret_cast<uintptr_t>(packed) % 16 != 0) return fail(DLP_INVALID_ARGUMENT, "packed weights must be 16-byte aligned");
     const long long total = (long long)L.n_pad * (L.k_pad / 4);
     const int threads = 256;
     const int blocks = int(std::min<long long>(ceil_div<long long>(total, threads), 8 * sm_count()));

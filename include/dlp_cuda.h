@@ -131,7 +131,7 @@ DLP_API size_t dlp_conv2d_fwd_workspace(const dlp_conv2d_plan *plan);
 /* Bytes of the pre-packed form of the weights (0 when the kernel reads raw weights). */
 DLP_API size_t dlp_conv2d_fwd_packed_bytes(const dlp_conv2d_plan *plan);
 /* Pack the weights once (TF32 hi/lo split into padded K-major tiles, or the Winograd filter
- * transform).  The reference redoes its filter transform on every call (src/core/conv.cpp:262-269);
+ * transform) into a 16-byte aligned buffer.  The reference redoes its filter transform on every call (src/core/conv.cpp:262-269);
  * inference weights are constant, so callers that own them can pack once and use enqueue_packed. */
 DLP_API dlp_status dlp_conv2d_fwd_prepack(const dlp_conv2d_plan *plan, const float *w, void *packed, void *stream);
 

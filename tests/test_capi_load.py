@@ -68,6 +68,11 @@ def test_argument_validation_needs_no_device():
         capi.check(capi.lib().dlp_tf32_issue_probe(4, 128, ctypes.byref(cycles), None))                # schemes are 0..3
     with pytest.raises(capi.ValidationError):
         capi.check(capi.lib().dlp_tf32_issue_probe(0, 96, ctypes.byref(cycles), None))                 # 64 or 128 columns
+    ip = capi.IPForward(64, 32, 1)
+    for call in (lambda: capi.lib().dlp_ip_fwd_prepack(ip.h, 1 << 20, (1 << 20) + 4, None),                     # packed forms are stored 16 bytes at a time
+                 lambda: capi.lib().dlp_ip_fwd_enqueue(ip.h, 1 << 20, 1 << 20, None, 1 << 20, (1 << 20) + 4, 1 << 20, 1, None)):
+        with pytest.raises(capi.ValidationError):
+            capi.check(call())
     assert capi.pooling2d_output_shape(112, 112, 3, 2, 1) == (56, 56)
     assert capi.pooling2d_output_shape(7, 7, 2, 2, 0, ceil_mode=True) == (4, 4)
     d = capi.make_conv_desc(channels_in=3, channels_out=64, kernel=7, stride=2, pad=3, height=224, width=224)
