@@ -192,8 +192,9 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *(volatile uint32_t *)&sh->tmem_base;
-    // (Each role waits for the kernel before, pdl_wait(), where it first touches global memory: barriers, tensor memory and the
-    // arithmetic of the first work item are done under that kernel.)
+    // (Each role waits for the kernel before, pdl_wait(), where it first touches global memory or waits for another role: barriers,
+    // tensor memory and the arithmetic of the first work item are done under that kernel, and the limit of a barrier wait counts
+    // from its end, whatever it takes.)
 
     // ---- epilogue pieces shared by the accumulate warps and, for a CTA's last work item, the loader warps
     // identity / relu / relu6 are a clamp; with no per-row bias and no beta the whole epilogue is
@@ -366,6 +367,7 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
         const int me = warp == WARP_MMA ? 0 : 1;
         uint32_t step = 0;
         bool dead = false;
+        pdl_wait();
         #pragma unroll 1
         while(it < total) {
             const uint32_t buf = chunk & 1;

@@ -164,7 +164,8 @@ pointwise_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *(volatile uint32_t *)&sh->tmem_base;
-    // (each role waits for the kernel before, pdl_wait(), where it first touches global memory)
+    // (each role waits for the kernel before, pdl_wait(), where it first touches global memory or waits for another role: the
+    // limit of a barrier wait counts from there, whatever the kernel before takes)
 
     if(warp == WARP_B) {
         // ------------------------------------------------------------------ B copies
@@ -257,6 +258,7 @@ pointwise_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
         uint32_t it = 0, step = 0, item_i = 0;
         int kb = 0;
         bool dead = false;
+        pdl_wait();
         #pragma unroll 1
         while(it < total) {
             const uint32_t s = it % T_STAGES, phase = (it / T_STAGES) & 1;
@@ -421,6 +423,7 @@ pointwise_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
         const int quad = warp & 3, group = (warp - WARP_CONV0) >> 2;
         const int row = quad * 32 + lane;
         const uint32_t total = uint32_t(my_items * kblocks);
+        pdl_wait();
         #pragma unroll 1
         for(uint32_t it = group; it < total; it += 2) {
             const int sa = it % S_STAGES, st = it % T_STAGES;

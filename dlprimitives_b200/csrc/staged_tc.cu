@@ -187,7 +187,8 @@ staged_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *(volatile uint32_t *)&sh->tmem_base;
-    // (each role waits for the kernel before, pdl_wait(), where it first touches global memory)
+    // (each role waits for the kernel before, pdl_wait(), where it first touches global memory or waits for another role: the
+    // limit of a barrier wait counts from there, whatever the kernel before takes)
 
     if(warp == WARP_A) {
         // ------------------------------------------------------------------ patch copies
@@ -256,6 +257,7 @@ staged_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
         int kb = 0, in_chunk = 0;
         const int me = warp == WARP_MMA ? 0 : 1;
         bool dead = false;
+        pdl_wait();
         #pragma unroll 1
         while(it < total) {
             const uint32_t buf = chunk & 1;
@@ -393,6 +395,7 @@ staged_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
         int kb = group;
         while(kb >= kblocks && patch0 < uint32_t(my_items) * q.cblocks) { kb -= kblocks; patch0 += q.cblocks; }
         uint32_t have_patch = 0xffffffffu;
+        pdl_wait();
         #pragma unroll 1
         for(uint32_t it = group; it < total; it += 2) {
             const uint32_t patch = patch0 + sh->kb_patch[kb];

@@ -201,7 +201,8 @@ stream_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const float *__re
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *(volatile uint32_t *)&sh->tmem_base;
-    // (each role waits for the kernel before, pdl_wait(), where it first touches global memory)
+    // (each role waits for the kernel before, pdl_wait(), where it first touches global memory or waits for another role: the
+    // limit of a barrier wait counts from there, whatever the kernel before takes)
 
     if(warp < WARP_ACC0) {
         regs_dec<REGS_ISSUE>();
@@ -298,6 +299,7 @@ stream_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const float *__re
             int kb = 0, in_chunk = 0;
             const int me = warp == WARP_MMA ? 0 : 1;
             bool dead = false;
+            pdl_wait();
             #pragma unroll 1
             while(it < total) {
                 const uint32_t buf = chunk & 1;
@@ -547,6 +549,7 @@ stream_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const float *__re
         float cur[BK], nxt[BK];
         bool have = false, release = false;
         uint32_t done = 0;
+        pdl_wait();
         #pragma unroll 1
         for(uint32_t it = group;; it += 2) {
             const bool more = it < total;
