@@ -121,11 +121,11 @@ __device__ __forceinline__ long long out_index(const Contraction &p, const RowIn
 
 __device__ __forceinline__ float finish_output(const Contraction &p, const RowInfo &r, long long row, int col, float acc)
 {
-    if(p.bias_mode == DLP_GEMM_BIAS_N) acc += __ldg(p.bias + col);
-    else if(p.bias_mode == DLP_GEMM_BIAS_M) acc += __ldg(p.bias + row);
+    if(p.bias_mode == DLP_GEMM_BIAS_N) acc += ld_plain(p.bias + col);
+    else if(p.bias_mode == DLP_GEMM_BIAS_M) acc += ld_plain(p.bias + row);
     acc = apply_act(acc, p.act);
     long long idx = out_index(p, r, col);
-    if(p.residual) acc = apply_act(acc + p.residual_scale * __ldg(p.residual + idx), p.post_act);
+    if(p.residual) acc = apply_act(acc + p.residual_scale * ld_plain(p.residual + idx), p.post_act);
     if(p.beta != 0.0f) acc += p.beta * p.y[idx];
     return acc;
 }

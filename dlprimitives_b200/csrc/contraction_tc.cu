@@ -78,16 +78,14 @@ struct Shared {
     uint32_t epilogue_started;   // work items of this CTA whose partial sums the accumulate warps have begun to read
 };
 
-// Lean store of N output columns of one row: y = clamp(acc + bias) [then clamp(y + s*residual)].
-template<int N, bool BIAS, bool RES>
-__device__ __forceinline__ void store_cols(const float (&v)[N], float *y0, const float (&res)[N], long long cs, const float *b0,
-                                           float2 clamp, float res_scale, float2 post_clamp, bool no_bias_loads = false, bool no_stg = false)
+// Lean store of N output columns of one row: y = clamp(v) [then clamp(y + s*residual)].
+template<int N, bool RES>
+__device__ __forceinline__ void store_cols(const float (&v)[N], float *y0, const float (&res)[N], long long cs, float2 clamp, float res_scale,
+                                           float2 post_clamp, bool no_stg = false)
 {
     #pragma unroll
     for(int j = 0; j < N; j++) {
-        float a = v[j];
-        if(BIAS) a += no_bias_loads ? 0.25f : __ldg(b0 + j);
-        a = fminf(fmaxf(a, clamp.x), clamp.y);
+        float a = fminf(fmaxf(v[j], clamp.x), clamp.y);
         if(RES) {
             a = a + res_scale * res[j];
             a = fminf(fmaxf(a, post_clamp.x), post_clamp.y);
@@ -127,7 +125,7 @@ struct Cursor {
 // parameter so that each kernel carries one loader only -- the roles share a small instruction cache.
 template<int BN, int MODE>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
-contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p, int kblocks, int n_tiles,
+contraction_tf32x3_kernel(const float *packed, const Contraction p, int kblocks, int n_tiles,
                           long long num_tiles, int splits, long long split_stride, int ktab_smem_entries, int *status, int diag,
                           long long *trace, const TcBatch batch)
 {
@@ -251,11 +249,16 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
         __syncwarp();
         if(warp == WARP_ACC0 && lane == 0) TC_TRACE(9, trace_idx);
         tmem_ld(taddr + g * G, v);
+        // the bias of a whole lean tile's columns, one a lane, handed round below
+        const int col0 = e.n0 + g * G;
+        const bool lean_bias = last && epi_fast && p.bias_mode == DLP_GEMM_BIAS_N && e.n0 + BN <= p.cols;      // warp-uniform
+        static_assert(G == 32, "a lane per column");
+        const float bias_lane = lean_bias ? (TC_DIAG(DIAG_NO_BIAS_LOADS) ? 0.25f : ld_plain(p.bias + col0 + lane)) : 0.0f;
         if(last && e.with_res) {
             // the residual operand of these columns travels while the tensor-memory load does
             const float *rp = e.res_row + (long long)(g * G) * e.col_stride;
             #pragma unroll
-            for(int j = 0; j < G; j++) { res[j] = TC_DIAG(DIAG_NO_RESIDUAL_LOADS) ? 0.5f : __ldg(rp); rp += e.col_stride; }
+            for(int j = 0; j < G; j++) { res[j] = TC_DIAG(DIAG_NO_RESIDUAL_LOADS) ? 0.5f : ld_plain(rp); rp += e.col_stride; }
         }
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         if(warp == WARP_ACC0 && lane == 0) TC_TRACE(10, trace_idx);
@@ -275,19 +278,15 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
             return;
         }
         // ---- last chunk: these columns of the row are final
-        const int col0 = e.n0 + g * G;
+        if(lean_bias) {
+            #pragma unroll
+            for(int j = 0; j < G; j++) x[j] += __shfl_sync(0xffffffffu, bias_lane, j);
+        }
         if(e.fast) {
             float *y0 = e.y_row + (long long)(g * G) * e.col_stride;
-            const float *b0 = p.bias + col0;
-            const bool nb = TC_DIAG(DIAG_NO_BIAS_LOADS), ns = TC_DIAG(DIAG_LEAN_NO_STG);
-            if(e.with_res) {
-                if(p.bias_mode == DLP_GEMM_BIAS_N) store_cols<G, true, true>(x, y0, res, e.col_stride, b0, clamp, p.residual_scale, post_clamp, nb, ns);
-                else store_cols<G, false, true>(x, y0, res, e.col_stride, b0, clamp, p.residual_scale, post_clamp, nb, ns);
-            }
-            else {
-                if(p.bias_mode == DLP_GEMM_BIAS_N) store_cols<G, true, false>(x, y0, res, e.col_stride, b0, clamp, 0.0f, post_clamp, nb, ns);
-                else store_cols<G, false, false>(x, y0, res, e.col_stride, b0, clamp, 0.0f, post_clamp, nb, ns);
-            }
+            const bool ns = TC_DIAG(DIAG_LEAN_NO_STG);
+            if(e.with_res) store_cols<G, true>(x, y0, res, e.col_stride, clamp, p.residual_scale, post_clamp, ns);
+            else store_cols<G, false>(x, y0, res, e.col_stride, clamp, 0.0f, post_clamp, ns);
         }
         else {
             // general epilogue: the values pass through the thread's own slots of the sums tile so
@@ -532,9 +531,9 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
                             #pragma unroll 1
                             for(int j = 0; j < ncols; j++) {
                                 float a = sg[j * BM];
-                                if(p.bias_mode == DLP_GEMM_BIAS_N) a += __ldg(p.bias + col0 + j);
+                                if(p.bias_mode == DLP_GEMM_BIAS_N) a += ld_plain(p.bias + col0 + j);
                                 a = fminf(fmaxf(a, clamp.x), clamp.y);
-                                if(r0) a = fminf(fmaxf(a + p.residual_scale * __ldg(r0 + (long long)j * col_stride), post_clamp.x), post_clamp.y);
+                                if(r0) a = fminf(fmaxf(a + p.residual_scale * ld_plain(r0 + (long long)j * col_stride), post_clamp.x), post_clamp.y);
                                 y0[(long long)j * col_stride] = a;
                             }
                         }
@@ -602,19 +601,19 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
                     const float4 *src4 = reinterpret_cast<const float4 *>(src);
                     #pragma unroll
                     for(int i = 0; i < BK / 4; i++) {
-                        const float4 t = __ldg(src4 + i);
+                        const float4 t = ld_plain(src4 + i);
                         buf[4 * i] = t.x; buf[4 * i + 1] = t.y; buf[4 * i + 2] = t.z; buf[4 * i + 3] = t.w;
                     }
                 }
                 else if(r.valid && k0 + BK <= p.k) {
                     #pragma unroll
-                    for(int i = 0; i < BK; i++) buf[i] = __ldg(src + (long long)i * p.a_k_stride);
+                    for(int i = 0; i < BK; i++) buf[i] = ld_plain(src + (long long)i * p.a_k_stride);
                 }
                 else {
                     #pragma unroll
                     for(int i = 0; i < BK; i++) {
                         const bool ok = r.valid && (k0 + i) < p.k;
-                        buf[i] = ok ? __ldg(src + (long long)i * p.a_k_stride) : 0.0f;
+                        buf[i] = ok ? ld_plain(src + (long long)i * p.a_k_stride) : 0.0f;
                     }
                 }
             }
@@ -624,7 +623,7 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
                 const float *src = p.a + r.base + (long long)(cb * BK) * p.a_k_stride + (d >> 16) * p.in_w + (d & 0xffff);
                 if(r.valid && unsigned(r.iy0 + (d >> 16)) < unsigned(p.in_h) && unsigned(r.ix0 + (d & 0xffff)) < unsigned(p.in_w)) {
                     #pragma unroll
-                    for(int i = 0; i < BK; i++) buf[i] = __ldg(src + (long long)i * p.a_k_stride);
+                    for(int i = 0; i < BK; i++) buf[i] = ld_plain(src + (long long)i * p.a_k_stride);
                 }
                 else {
                     #pragma unroll
@@ -641,7 +640,7 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
                     const float *src = p.a + r.base + e.x;
                     const unsigned cols = ((row_mask >> e.y) & 1u) ? col_mask : 0u;
                     #pragma unroll
-                    for(int kx = 0; kx < ROWTAPS_WIDTH; kx++) buf[g * ROWTAPS_WIDTH + kx] = (cols >> kx) & 1u ? __ldg(src + kx) : 0.0f;
+                    for(int kx = 0; kx < ROWTAPS_WIDTH; kx++) buf[g * ROWTAPS_WIDTH + kx] = (cols >> kx) & 1u ? ld_plain(src + kx) : 0.0f;
                 }
             }
             else {
@@ -657,8 +656,8 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
                         for(int j = 0; j < 4; j++) e[j] = tab[i0 / 2 + j];
                         #pragma unroll
                         for(int j = 0; j < 4; j++) {
-                            buf[i0 + 2 * j] = tap_inside(e[j].y) ? __ldg(src + e[j].x) : 0.0f;
-                            buf[i0 + 2 * j + 1] = tap_inside(e[j].w) ? __ldg(src + e[j].z) : 0.0f;
+                            buf[i0 + 2 * j] = tap_inside(e[j].y) ? ld_plain(src + e[j].x) : 0.0f;
+                            buf[i0 + 2 * j + 1] = tap_inside(e[j].w) ? ld_plain(src + e[j].z) : 0.0f;
                         }
                     }
                 }
@@ -668,7 +667,7 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
                     for(int i = 0; i < BK; i++) {
                         const int2 t = __ldg(tab + i);          // offset, tap number (63 = padding beyond K: never valid)
                         const bool ok = tap_inside(t.y);
-                        buf[i] = ok ? __ldg(src + t.x) : 0.0f;
+                        buf[i] = ok ? ld_plain(src + t.x) : 0.0f;
                     }
                 }
             }
@@ -784,7 +783,7 @@ contraction_tf32x3_kernel(const float *__restrict__ packed, const Contraction p,
 // otherwise consecutive threads take consecutive chunks along k (sources whose k is contiguous, read 16 bytes at a time when aligned).
 // Index: unsigned when the chunks of a matrix are fewer than 2^31 (a 64-bit division per chunk cost more than its bytes).
 template<typename Index>
-__global__ void prepack_kernel(const float *__restrict__ b, long long col_stride, long long k_stride, int cols, int k,
+__global__ void prepack_kernel(const float *b, long long col_stride, long long k_stride, int cols, int k,
                                int n_pad, int k_pad, int bn, int taps, float *__restrict__ packed, long long b_batch_stride, int n_major,
                                int row_kw)
 {
@@ -810,7 +809,7 @@ __global__ void prepack_kernel(const float *__restrict__ b, long long col_stride
         float v[4] = { 0.0f, 0.0f, 0.0f, 0.0f };
         if(n < cols) {
             if(vec && kk + 4 <= k) {
-                const float4 t = __ldg(reinterpret_cast<const float4 *>(b + n * col_stride + kk));
+                const float4 t = ld_plain(reinterpret_cast<const float4 *>(b + n * col_stride + kk));
                 v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
             }
             else {
@@ -829,7 +828,7 @@ __global__ void prepack_kernel(const float *__restrict__ b, long long col_stride
                         ks = g * row_kw + kx;
                         exists = kx < row_kw && ks < k;
                     }
-                    if(exists) v[j] = __ldg(b + n * col_stride + ks * k_stride);
+                    if(exists) v[j] = ld_plain(b + n * col_stride + ks * k_stride);
                 }
             }
         }
@@ -852,7 +851,7 @@ __global__ void prepack_kernel(const float *__restrict__ b, long long col_stride
 // one element at a time, part after part, the trips to L2 added up (sixteen parts of a 1 x 1000 result took longer than the
 // products; two parts of a 3136 x 1024 one moved 1.4 TB/s).  Index arithmetic in 32 bits when the quads are fewer than 2^31.
 template<typename Index>
-__global__ void __launch_bounds__(256) split_finish_kernel(const Contraction p, const float *__restrict__ partial, int splits,
+__global__ void __launch_bounds__(256) split_finish_kernel(const Contraction p, const float *partial, int splits,
                                                            long long split_stride, long long rows_pad)
 {
     pdl_wait();
@@ -861,13 +860,13 @@ __global__ void __launch_bounds__(256) split_finish_kernel(const Contraction p, 
         const int col = int(idx / quads);
         const long long row = 4 * (long long)(idx - Index(col) * quads);
         const float *src = partial + (long long)col * rows_pad + row;
-        float4 acc = __ldg(reinterpret_cast<const float4 *>(src));
+        float4 acc = ld_plain(reinterpret_cast<const float4 *>(src));
         #pragma unroll 1
         for(int s = 1; s < splits; s += 8) {
             float4 v[8];
             #pragma unroll
             for(int j = 0; j < 8; j++)
-                if(s + j < splits) v[j] = __ldg(reinterpret_cast<const float4 *>(src + (s + j) * split_stride));
+                if(s + j < splits) v[j] = ld_plain(reinterpret_cast<const float4 *>(src + (s + j) * split_stride));
             #pragma unroll
             for(int j = 0; j < 8; j++)
                 if(s + j < splits) { acc.x += v[j].x; acc.y += v[j].y; acc.z += v[j].z; acc.w += v[j].w; }
@@ -877,6 +876,9 @@ __global__ void __launch_bounds__(256) split_finish_kernel(const Contraction p, 
         // the four rows follow each other in y when they are pixels of one image, or y is column-major
         const bool together = p.out_mode == OUT_COL_MAJOR || (p.out_mode == OUT_NCHW && p.plane % 4 == 0);
         const long long step = p.out_mode == OUT_ROW_MAJOR ? p.ldc : 1;
+        // bias, residual and old values of all four first: behind the first store their loads would go one after the other
+        long long at[4];
+        float out[4];
         #pragma unroll
         for(int j = 0; j < 4; j++) {
             if(row + j >= p.rows) break;
@@ -884,7 +886,13 @@ __global__ void __launch_bounds__(256) split_finish_kernel(const Contraction p, 
                 if(together || p.out_mode == OUT_ROW_MAJOR) r.out += step;
                 else r = make_row(p, row + j);
             }
-            p.y[out_index(p, r, col)] = finish_output(p, r, row + j, col, a[j]);
+            at[j] = out_index(p, r, col);
+            out[j] = finish_output(p, r, row + j, col, a[j]);
+        }
+        #pragma unroll
+        for(int j = 0; j < 4; j++) {
+            if(row + j >= p.rows) break;
+            p.y[at[j]] = out[j];
         }
     }
 }

@@ -63,15 +63,15 @@ __global__ void __launch_bounds__(THREADS) depthwise_kernel(DwParams p)
         for(; i + (U - 1) * THREADS * 4 < safe; i += U * THREADS * 4) {
             float4 v[U];
             #pragma unroll
-            for(int u = 0; u < U; u++) v[u] = __ldg(reinterpret_cast<const float4 *>(p.x + a_begin + i + u * THREADS * 4));
+            for(int u = 0; u < U; u++) v[u] = ld_plain(reinterpret_cast<const float4 *>(p.x + a_begin + i + u * THREADS * 4));
             #pragma unroll
             for(int u = 0; u < U; u++) *reinterpret_cast<float4 *>(tile + i + u * THREADS * 4) = v[u];
         }
         for(; i < count; i += THREADS * 4) {
             const long long gi = a_begin + i;
-            if(i + 4 <= safe) *reinterpret_cast<float4 *>(tile + i) = __ldg(reinterpret_cast<const float4 *>(p.x + gi));
+            if(i + 4 <= safe) *reinterpret_cast<float4 *>(tile + i) = ld_plain(reinterpret_cast<const float4 *>(p.x + gi));
             else
-                for(int j = 0; j < 4 && gi + j < total_in; j++) tile[i + j] = __ldg(p.x + gi + j);
+                for(int j = 0; j < 4 && gi + j < total_in; j++) tile[i + j] = ld_plain(p.x + gi + j);
         }
     }
     __syncthreads();
@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(THREADS) depthwise_kernel(DwParams p)
             const int c = int(plane % p.channels);
             float wreg[(KS > 0 ? KS : 1) * (KS > 0 ? KS : 1)];
             #pragma unroll
-            for(int i = 0; i < KS * KS; i++) wreg[i] = __ldg(p.w + (long long)c * (KS * KS) + i);
+            for(int i = 0; i < KS * KS; i++) wreg[i] = ld_plain(p.w + (long long)c * (KS * KS) + i);
             const int ox0 = oxp * CW, nc = min(CW, p.OW - ox0);
             const int oyb = oy0 + seg * R, nr = min(R, oy1 - oyb);
             const int iyb = oyb * ST - p.pad, ix0 = ox0 * ST - p.pad;
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(THREADS) depthwise_kernel(DwParams p)
                             if((col_ok >> (cc * ST + kx)) & 1u) acc[j][cc] = fmaf(v[cc * ST + kx], wreg[ky * KS + kx], acc[j][cc]);
                 }
             }
-            const float b = p.bias ? __ldg(p.bias + c) : 0.0f;
+            const float b = p.bias ? ld_plain(p.bias + c) : 0.0f;
             #pragma unroll
             for(int j = 0; j < R; j++) {
                 if(j >= nr) break;
@@ -164,10 +164,10 @@ __global__ void __launch_bounds__(THREADS) depthwise_kernel(DwParams p)
             for(int kx = 0; kx < ks; kx++) {
                 const int ix = ix0 + kx;
                 if(unsigned(ix) >= unsigned(p.W)) continue;
-                acc = fmaf(src[iy * p.W + ix], __ldg(wk + ky * ks + kx), acc);
+                acc = fmaf(src[iy * p.W + ix], ld_plain(wk + ky * ks + kx), acc);
             }
         }
-        if(p.bias) acc += __ldg(p.bias + c);
+        if(p.bias) acc += ld_plain(p.bias + c);
         acc = apply_act(acc, p.act);
         const long long yi = plane * ((long long)p.OH * p.OW) + (long long)oy * p.OW + ox;
         if(p.factor != 0.0f) acc += p.factor * p.y[yi];
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(THREADS) depthwise3_reg_kernel(DwParams p, lon
     const float *xin = p.x + pl * ((long long)p.H * p.W) + c * V;
     float w[9];
     #pragma unroll
-    for(int i = 0; i < 9; i++) w[i] = valid ? __ldg(p.w + ch * 9 + i) : 0.0f;
+    for(int i = 0; i < 9; i++) w[i] = valid ? ld_plain(p.w + ch * 9 + i) : 0.0f;
 
     float in[RI][V + 2];     // [0]: the column to the left, [1..V]: the lane's own, [V+1]: the column to the right (stride 1)
     bool ok[RI];
@@ -213,16 +213,16 @@ __global__ void __launch_bounds__(THREADS) depthwise3_reg_kernel(DwParams p, lon
         ok[i] = valid && iy >= 0 && iy < p.H;
         const float *row = xin + (long long)iy * p.W;
         if(V == 4) {
-            const float4 t = ok[i] ? __ldg(reinterpret_cast<const float4 *>(row)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float4 t = ok[i] ? ld_plain(reinterpret_cast<const float4 *>(row)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             in[i][1] = t.x; in[i][2] = t.y; in[i][3] = t.z; in[i][4] = t.w;
         }
         else {
-            const float2 t = ok[i] ? __ldg(reinterpret_cast<const float2 *>(row)) : make_float2(0.0f, 0.0f);
+            const float2 t = ok[i] ? ld_plain(reinterpret_cast<const float2 *>(row)) : make_float2(0.0f, 0.0f);
             in[i][1] = t.x; in[i][2] = t.y;
         }
         // the first and the last lane of the warp have their neighbour in another warp: one more load
-        in[i][0] = (ok[i] && lane == 0 && c > 0) ? __ldg(row - 1) : 0.0f;
-        in[i][V + 1] = (S == 1 && ok[i] && lane == 31 && c < qw - 1) ? __ldg(row + V) : 0.0f;
+        in[i][0] = (ok[i] && lane == 0 && c > 0) ? ld_plain(row - 1) : 0.0f;
+        in[i][V + 1] = (S == 1 && ok[i] && lane == 31 && c < qw - 1) ? ld_plain(row + V) : 0.0f;
     }
     #pragma unroll
     for(int i = 0; i < RI; i++) {
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(THREADS) depthwise3_reg_kernel(DwParams p, lon
         if(S == 1 && lane < 31) in[i][V + 1] = c < qw - 1 ? from_right : 0.0f;
     }
     if(!valid) return;
-    const float b = p.bias ? __ldg(p.bias + ch) : 0.0f;
+    const float b = p.bias ? ld_plain(p.bias + ch) : 0.0f;
     float *yrow = p.y + pl * ((long long)p.OH * p.OW) + c * VO;
     #pragma unroll
     for(int j = 0; j < RS; j++) {
@@ -285,17 +285,17 @@ __global__ void __launch_bounds__(THREADS) depthwise3_rows_kernel(DwParams p, lo
     if(W % 2 == 0) {
         #pragma unroll
         for(int i = 0; i < W / 2; i++) {
-            const float2 t = have ? __ldg(reinterpret_cast<const float2 *>(src) + i) : make_float2(0.0f, 0.0f);
+            const float2 t = have ? ld_plain(reinterpret_cast<const float2 *>(src) + i) : make_float2(0.0f, 0.0f);
             in[1 + 2 * i] = t.x; in[2 + 2 * i] = t.y;
         }
     }
     else {
         #pragma unroll
-        for(int i = 0; i < W; i++) in[1 + i] = have ? __ldg(src + i) : 0.0f;
+        for(int i = 0; i < W; i++) in[1 + i] = have ? ld_plain(src + i) : 0.0f;
     }
     float w[9];
     #pragma unroll
-    for(int i = 0; i < 9; i++) w[i] = have ? __ldg(p.w + ch * 9 + i) : 0.0f;
+    for(int i = 0; i < 9; i++) w[i] = have ? ld_plain(p.w + ch * 9 + i) : 0.0f;
     float up[W + 2], down[W + 2];
     up[0] = up[W + 1] = down[0] = down[W + 1] = 0.0f;
     const bool has_up = r > 0, has_down = r < p.H - 1;
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(THREADS) depthwise3_rows_kernel(DwParams p, lo
     if(!have || lane == 0 || lane == 31 || (S == 2 && (r & 1))) return;
     const int orow = S == 1 ? r : r / 2;
     if(orow >= p.OH) return;
-    const float b = p.bias ? __ldg(p.bias + ch) : 0.0f;
+    const float b = p.bias ? ld_plain(p.bias + ch) : 0.0f;
     float *dst = p.y + (plane * p.OH + orow) * (long long)p.OW;
     float o[OWC];
     #pragma unroll
@@ -347,17 +347,20 @@ __global__ void __launch_bounds__(THREADS) depthwise1_scale_kernel(DwParams p, u
     constexpr int U = 4;
     const unsigned nthreads = gridDim.x * blockDim.x;
     for(unsigned g0 = blockIdx.x * blockDim.x + threadIdx.x; g0 < total4; g0 += U * nthreads) {
-        float v[U][4];
+        float v[U][4], w0[U], b0[U];       // (weight and bias of the first element's plane: of all four when vec)
         #pragma unroll
         for(int u = 0; u < U; u++) {
             const unsigned g = g0 + u * nthreads;
             if(g >= total4) continue;
+            const unsigned c = ((4 * g) / unsigned(plane)) % unsigned(p.channels);
+            w0[u] = ld_plain(p.w + c);
+            b0[u] = p.bias ? ld_plain(p.bias + c) : 0.0f;
             if(vec) {
-                const float4 t = __ldg(reinterpret_cast<const float4 *>(p.x) + g);
+                const float4 t = ld_plain(reinterpret_cast<const float4 *>(p.x) + g);
                 v[u][0] = t.x; v[u][1] = t.y; v[u][2] = t.z; v[u][3] = t.w;
             }
             else
-                for(int j = 0; j < 4; j++) v[u][j] = 4 * g + j < total ? __ldg(p.x + 4 * g + j) : 0.0f;
+                for(int j = 0; j < 4; j++) v[u][j] = 4 * g + j < total ? ld_plain(p.x + 4 * g + j) : 0.0f;
         }
         #pragma unroll
         for(int u = 0; u < U; u++) {
@@ -365,14 +368,13 @@ __global__ void __launch_bounds__(THREADS) depthwise1_scale_kernel(DwParams p, u
             if(g >= total4) continue;
             float o[4];
             // vec: the four elements lie in one plane and share its weight and bias
-            unsigned c = ((4 * g) / unsigned(plane)) % unsigned(p.channels);
-            float wc = __ldg(p.w + c), bc = p.bias ? __ldg(p.bias + c) : 0.0f;
+            float wc = w0[u], bc = b0[u];
             #pragma unroll
             for(int j = 0; j < 4; j++) {
                 if(!vec && j > 0) {
-                    c = ((4 * g + j) / unsigned(plane)) % unsigned(p.channels);
-                    wc = __ldg(p.w + c);
-                    bc = p.bias ? __ldg(p.bias + c) : 0.0f;
+                    const unsigned c = ((4 * g + j) / unsigned(plane)) % unsigned(p.channels);
+                    wc = ld_plain(p.w + c);
+                    bc = p.bias ? ld_plain(p.bias + c) : 0.0f;
                 }
                 float a = fmaf(v[u][j], wc, 0.0f);
                 if(p.bias) a += bc;

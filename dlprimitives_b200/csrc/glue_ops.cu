@@ -7,7 +7,7 @@
 namespace dlp {
 namespace {
 
-__global__ void pooling2d_kernel(const float *__restrict__ x, float *__restrict__ y, long long total, int in_h, int in_w, int out_h,
+__global__ void pooling2d_kernel(const float *x, float *__restrict__ y, long long total, int in_h, int in_w, int out_h,
                                  int out_w, int kh, int kw, int sh, int sw, int ph, int pw, int mode_avg, int include_pad)
 {
     pdl_wait();
@@ -26,7 +26,7 @@ __global__ void pooling2d_kernel(const float *__restrict__ x, float *__restrict_
         float val = mode_avg ? 0.0f : -FLT_MAX;
         for(int r = row0; r < row1; r++)
             for(int c = col0; c < col1; c++) {
-                const float v = __ldg(src + r * in_w + c);
+                const float v = ld_plain(src + r * in_w + c);
                 val = mode_avg ? val + v : fmaxf(val, v);
             }
         if(mode_avg) {
@@ -44,7 +44,7 @@ __global__ void pooling2d_kernel(const float *__restrict__ x, float *__restrict_
 // from shared memory.  The arithmetic is the same as pooling2d_kernel's, in the same order.
 // K, S: kernel size and stride when square and known at compile time (the window loops unroll), 0 = run-time values.
 template<int K, int S>
-__global__ void pooling2d_band_kernel(const float *__restrict__ x, float *__restrict__ y, long long bands_total, int bands_per_plane,
+__global__ void pooling2d_band_kernel(const float *x, float *__restrict__ y, long long bands_total, int bands_per_plane,
                                       int band_rows, int in_h, int in_w, int out_h, int out_w, int kh_, int kw_, int sh_, int sw_, int ph,
                                       int pw, int mode_avg, int include_pad, int vec_ok)
 {
@@ -62,10 +62,10 @@ __global__ void pooling2d_band_kernel(const float *__restrict__ x, float *__rest
             // in_w is a multiple of 4 and x is 16-byte aligned, so every row starts on a 16-byte boundary
             const float4 *src4 = reinterpret_cast<const float4 *>(src);
             float4 *tile4 = reinterpret_cast<float4 *>(tile);
-            for(int i = threadIdx.x; i < count / 4; i += blockDim.x) tile4[i] = __ldg(src4 + i);
+            for(int i = threadIdx.x; i < count / 4; i += blockDim.x) tile4[i] = ld_plain(src4 + i);
         }
         else
-            for(int i = threadIdx.x; i < count; i += blockDim.x) tile[i] = __ldg(src + i);
+            for(int i = threadIdx.x; i < count; i += blockDim.x) tile[i] = ld_plain(src + i);
         __syncthreads();
         float *dst = y + plane * (long long)out_h * out_w + (long long)orow0 * out_w;
         for(int i = threadIdx.x; i < orows * out_w; i += blockDim.x) {
@@ -115,7 +115,7 @@ __global__ void pooling2d_band_kernel(const float *__restrict__ x, float *__rest
 // keeps the row maxima in registers; all the strip's loads are issued before the first is used.  Maximum is exact in any
 // order, so the result is bit-identical to pooling2d_kernel's.
 template<int RS>
-__global__ void __launch_bounds__(256) pool_max3s2_kernel(const float *__restrict__ x, float *__restrict__ y, long long items, int col_blocks,
+__global__ void __launch_bounds__(256) pool_max3s2_kernel(const float *x, float *__restrict__ y, long long items, int col_blocks,
                                                           int strips, int in_h, int in_w, int out_h, int out_w)
 {
     pdl_wait();
@@ -136,9 +136,9 @@ __global__ void __launch_bounds__(256) pool_max3s2_kernel(const float *__restric
     for(int r = 0; r < ROWS; r++) {
         const int iy = 2 * orow0 - 1 + r;
         const bool ok = col_ok && iy >= 0 && iy < in_h;
-        a[r] = ok ? __ldg(reinterpret_cast<const float2 *>(src + (long long)iy * in_w) + oc) : make_float2(-FLT_MAX, -FLT_MAX);
+        a[r] = ok ? ld_plain(reinterpret_cast<const float2 *>(src + (long long)iy * in_w) + oc) : make_float2(-FLT_MAX, -FLT_MAX);
         // lane 0 has no left neighbour in the warp: column 2*oc-1 is the padding (first block) or one more load
-        left[r] = (ok && lane == 0 && oc > 0) ? __ldg(src + (long long)iy * in_w + 2 * oc - 1) : -FLT_MAX;
+        left[r] = (ok && lane == 0 && oc > 0) ? ld_plain(src + (long long)iy * in_w + 2 * oc - 1) : -FLT_MAX;
     }
     float h[ROWS];
     #pragma unroll
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(256) pool_max3s2_kernel(const float *__restric
 
 // Global pooling of small odd-sized planes: a CTA of 128 threads copies 128 consecutive planes into shared memory with
 // coalesced 16-byte loads, then thread t reduces plane t in index order (odd plane size: conflict-free).
-__global__ void __launch_bounds__(128) global_pooling_tile_kernel(const float *__restrict__ x, float *__restrict__ y, int planes, int plane_size,
+__global__ void __launch_bounds__(128) global_pooling_tile_kernel(const float *x, float *__restrict__ y, int planes, int plane_size,
                                                                   int mode_avg)
 {
     pdl_wait();
@@ -164,8 +164,8 @@ __global__ void __launch_bounds__(128) global_pooling_tile_kernel(const float *_
     const float *src = x + (long long)plane0 * plane_size;           // 128 * plane_size * 4 bytes per CTA: 16-byte aligned when x is
     const float4 *src4 = reinterpret_cast<const float4 *>(src);
     float4 *tile4 = reinterpret_cast<float4 *>(tile);
-    for(int i = threadIdx.x; i < count / 4; i += 128) tile4[i] = __ldg(src4 + i);
-    for(int i = (count & ~3) + threadIdx.x; i < count; i += 128) tile[i] = __ldg(src + i);
+    for(int i = threadIdx.x; i < count / 4; i += 128) tile4[i] = ld_plain(src4 + i);
+    for(int i = (count & ~3) + threadIdx.x; i < count; i += 128) tile[i] = ld_plain(src + i);
     __syncthreads();
     if(plane0 + int(threadIdx.x) >= planes) return;
     const float *mine = tile + threadIdx.x * plane_size;
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(128) global_pooling_tile_kernel(const float *_
 }
 
 // one warp per plane
-__global__ void global_pooling_kernel(const float *__restrict__ x, float *__restrict__ y, int planes, int plane_size, int mode_avg)
+__global__ void global_pooling_kernel(const float *x, float *__restrict__ y, int planes, int plane_size, int mode_avg)
 {
     pdl_wait();
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
@@ -183,7 +183,7 @@ __global__ void global_pooling_kernel(const float *__restrict__ x, float *__rest
     const float *src = x + (long long)warp * plane_size;
     float v = mode_avg ? 0.0f : -FLT_MAX;
     for(int i = lane; i < plane_size; i += 32) {
-        const float a = __ldg(src + i);
+        const float a = ld_plain(src + i);
         v = mode_avg ? v + a : fmaxf(v, a);
     }
     #pragma unroll
@@ -283,18 +283,18 @@ __global__ void softmax_kernel(const float *x, float *y, int classes, int inner,
 // y may be x (in place).
 template<typename Index>
 __global__ void __launch_bounds__(256) batchnorm_inference_kernel(const float *x, float *y, Index count, Index features, Index plane, float eps,
-                                                                  const float *__restrict__ mean, const float *__restrict__ var,
-                                                                  const float *__restrict__ gamma, const float *__restrict__ beta, int vec_ok)
+                                                                  const float *mean, const float *var,
+                                                                  const float *gamma, const float *beta, int vec_ok)
 {
     pdl_wait();
     auto coefficients = [&](Index i) {
         const Index f = (i / plane) % features;
-        float a = 1.0f / sqrtf(__ldg(var + f) + eps);
-        float b = -__ldg(mean + f) * a;
+        float a = 1.0f / sqrtf(ld_plain(var + f) + eps);
+        float b = -ld_plain(mean + f) * a;
         if(gamma && beta) {
-            const float g = __ldg(gamma + f);
+            const float g = ld_plain(gamma + f);
             a *= g;
-            b = g * b + __ldg(beta + f);
+            b = g * b + ld_plain(beta + f);
         }
         return make_float2(a, b);
     };

@@ -125,7 +125,7 @@ __device__ __forceinline__ void drain_own(unsigned long long *bars, int depth, u
 template<int BN>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 pointwise_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_y,
-                        const __grid_constant__ CUtensorMap tm_res, const float *__restrict__ packed, const Params q, int *status)
+                        const __grid_constant__ CUtensorMap tm_res, const float *packed, const Params q, int *status)
 {
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -345,7 +345,7 @@ pointwise_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
             #pragma unroll
             for(int u = 0; u < 2; u++) {
                 const int col = w.n_tile * BN + (set + u * SETS) * 32 + lane;
-                if(set + u * SETS < GROUPS && q.bias && col < q.cols) bias_g[u] = ldg_early(q.bias + col);
+                if(set + u * SETS < GROUPS && q.bias && col < q.cols) bias_g[u] = ld_early(q.bias + col);
             }
             // A wait that gives up must not leave the other epilogue warps alone at the block barrier below: a warp
             // that failed keeps walking the groups without touching anything, and the barrier itself carries the

@@ -132,7 +132,7 @@ __device__ __forceinline__ void tma_load_4d(void *dst, const void *tmap, int x, 
 
 template<int BN>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
-staged_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_y, const float *__restrict__ packed,
+staged_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_y, const float *packed,
                      const Params q, int *status)
 {
     extern __shared__ unsigned char smem_raw[];
@@ -336,7 +336,7 @@ staged_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
         for(long long item = blockIdx.x; item < q.num_items && live; item += gridDim.x, i++) {
             const Item w = decode(item, q);
             // the bias of the set's 32 channels is asked for now: its trip to L2 is over long before the last chunk is in
-            const float bias_lane = q.bias && w.n_tile * BN + g * 32 + lane < q.cols ? ldg_early(q.bias + w.n_tile * BN + g * 32 + lane) : 0.0f;
+            const float bias_lane = q.bias && w.n_tile * BN + g * 32 + lane < q.cols ? ld_early(q.bias + w.n_tile * BN + g * 32 + lane) : 0.0f;
             float sum[32];
             bool ok = true;
             #pragma unroll 1

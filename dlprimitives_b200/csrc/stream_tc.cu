@@ -156,7 +156,7 @@ template<int R> __device__ __forceinline__ void regs_dec() { asm volatile("setma
 // SRC: how A lies in memory and comes in (see the top of the file).
 template<int BN, int SRC>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
-stream_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const float *__restrict__ packed, const Params q, int *status)
+stream_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const float *packed, const Params q, int *status)
 {
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -391,7 +391,7 @@ stream_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const float *__re
                 float bias_g[COLS / 32];
                 #pragma unroll
                 for(int g = 0; g < COLS / 32; g++)
-                    bias_g[g] = q.bias && col0 + g * 32 + lane < q.cols ? ldg_early(q.bias + col0 + g * 32 + lane) : 0.0f;
+                    bias_g[g] = q.bias && col0 + g * 32 + lane < q.cols ? ld_early(q.bias + col0 + g * 32 + lane) : 0.0f;
                 if(q.residual) {
                     // each lane sees to two columns: the warp's first and last row (a column of the warp is one or two lines)
                     const long long first = __shfl_sync(0xffffffffu, off, 0), lastv = __shfl_sync(0xffffffffu, valid ? off : first, 31);
@@ -432,7 +432,7 @@ stream_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const float *__re
                 auto load_res = [&](int h) {
                     #pragma unroll
                     for(int j = 0; j < 8; j++) {
-                        res[h & 1][j] = res_ok && h * 8 + j < cols_left ? __ldg(rp) : 0.0f;
+                        res[h & 1][j] = res_ok && h * 8 + j < cols_left ? ld_plain(rp) : 0.0f;
                         rp += q.y_col_stride;
                     }
                 };

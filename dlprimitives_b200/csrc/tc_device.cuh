@@ -107,12 +107,12 @@ __device__ __forceinline__ bool warp_wait_ready(unsigned long long *bar, uint32_
     return warp_wait(bar, parity, abort_flag, status, code, lane);
 }
 
-// A read-only load that stays where it is written (the compiler keeps it ahead of the waits that follow): for operands
-// asked for early so that their trip to L2 is over by the time they are used.
-__device__ __forceinline__ float ldg_early(const float *p)
+// A load that stays where it is written (the compiler keeps it ahead of the waits that follow): for operands asked for early so
+// that their trip to L2 is over by the time they are used.  Plain, as ld_plain.
+__device__ __forceinline__ float ld_early(const float *p)
 {
     float v;
-    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
     return v;
 }
 

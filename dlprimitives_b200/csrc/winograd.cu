@@ -25,7 +25,7 @@ constexpr int WC = 8;         // input channels per step
 constexpr int WTHREADS = 256;
 
 // U[xi][c][o] = (G g G^T)[xi] for filter (o, c); o padded to cout_pad with zeros
-__global__ void winograd_filter_transform_kernel(const float *__restrict__ w, float *__restrict__ u, int cin, int cout, int cout_pad)
+__global__ void winograd_filter_transform_kernel(const float *w, float *__restrict__ u, int cin, int cout, int cout_pad)
 {
     pdl_wait();
     const long long total = (long long)cin * cout_pad;
@@ -35,7 +35,7 @@ __global__ void winograd_filter_transform_kernel(const float *__restrict__ w, fl
         #pragma unroll
         for(int i = 0; i < 3; i++)
             #pragma unroll
-            for(int j = 0; j < 3; j++) g[i][j] = o < cout ? __ldg(w + ((long long)o * cin + c) * 9 + i * 3 + j) : 0.0f;
+            for(int j = 0; j < 3; j++) g[i][j] = o < cout ? ld_plain(w + ((long long)o * cin + c) * 9 + i * 3 + j) : 0.0f;
         float t[4][3];     // G g
         #pragma unroll
         for(int j = 0; j < 3; j++) {

@@ -22,14 +22,14 @@ namespace dlp {
 namespace {
 
 // Uraw[xi][o][c] = (G g G^T)[xi] for filter (o, c)
-__global__ void wtc_filter_kernel(const float *__restrict__ w, float *__restrict__ u, int cin, int cout)
+__global__ void wtc_filter_kernel(const float *w, float *__restrict__ u, int cin, int cout)
 {
     pdl_wait();
     const long long total = (long long)cin * cout;
     for(long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
         float g[3][3];
         #pragma unroll
-        for(int i = 0; i < 9; i++) g[i / 3][i % 3] = __ldg(w + idx * 9 + i);          // idx = o * cin + c
+        for(int i = 0; i < 9; i++) g[i / 3][i % 3] = ld_plain(w + idx * 9 + i);          // idx = o * cin + c
         float t[4][3];
         #pragma unroll
         for(int j = 0; j < 3; j++) {
@@ -55,7 +55,7 @@ struct Geometry {
 // one thread per (channel plane, tile): reads the 4x4 patch, writes the 16 transformed values (tiles contiguous across lanes).
 // Index: unsigned when (channel, tile) pairs fit 31 bits -- three 64-bit divisions per patch cost more than its bytes.
 template<typename Index>
-__global__ void wtc_input_kernel(const float *__restrict__ x, float *__restrict__ v, Geometry q)
+__global__ void wtc_input_kernel(const float *x, float *__restrict__ v, Geometry q)
 {
     pdl_wait();
     const Index per_image = Index(q.tiles_h) * Index(q.tiles_w), tiles = Index(q.tiles), total = tiles * Index(q.cin);
@@ -72,7 +72,7 @@ __global__ void wtc_input_kernel(const float *__restrict__ x, float *__restrict_
             #pragma unroll
             for(int j = 0; j < 4; j++) {
                 const int ix = 2 * tx - 1 + j;
-                d[i][j] = (unsigned(iy) < unsigned(q.h) && unsigned(ix) < unsigned(q.w)) ? __ldg(src + (long long)iy * q.w + ix) : 0.0f;
+                d[i][j] = (unsigned(iy) < unsigned(q.h) && unsigned(ix) < unsigned(q.w)) ? ld_plain(src + (long long)iy * q.w + ix) : 0.0f;
             }
         }
         float m[4][4];     // B^T d
@@ -104,7 +104,7 @@ struct OutArgs {
 
 // one thread per (output channel plane, tile): reads the 16 products, writes the 2x2 outputs
 template<typename Index>
-__global__ void wtc_output_kernel(const float *__restrict__ mm, Geometry q, OutArgs a)
+__global__ void wtc_output_kernel(const float *mm, Geometry q, OutArgs a)
 {
     pdl_wait();
     const Index per_image = Index(q.tiles_h) * Index(q.tiles_w), tiles = Index(q.tiles), total = tiles * Index(q.cout);
@@ -117,14 +117,22 @@ __global__ void wtc_output_kernel(const float *__restrict__ mm, Geometry q, OutA
         const long long xi_stride = (long long)q.cout * q.tiles_pad;
         float m[4][4];
         #pragma unroll
-        for(int i = 0; i < 16; i++) m[i / 4][i % 4] = __ldg(src + i * xi_stride);
+        for(int i = 0; i < 16; i++) m[i / 4][i % 4] = ld_plain(src + i * xi_stride);
         float s[2][4];     // A^T M
         #pragma unroll
         for(int j = 0; j < 4; j++) {
             s[0][j] = m[0][j] + m[1][j] + m[2][j];
             s[1][j] = m[1][j] - m[2][j] - m[3][j];
         }
-        const float bias = a.bias ? __ldg(a.bias + o) : 0.0f;
+        const float bias = a.bias ? ld_plain(a.bias + o) : 0.0f;
+        // the residual of all four outputs ahead of the first store
+        const long long y0 = (((long long)b * q.cout + o) * q.h + 2 * ty) * q.w + 2 * tx;
+        float res[2][2];
+        #pragma unroll
+        for(int i = 0; i < 2; i++)
+            #pragma unroll
+            for(int j = 0; j < 2; j++)
+                res[i][j] = a.residual && 2 * ty + i < q.h && 2 * tx + j < q.w ? ld_plain(a.residual + y0 + (long long)i * q.w + j) : 0.0f;
         #pragma unroll
         for(int i = 0; i < 2; i++) {
             const int oy = 2 * ty + i;
@@ -134,9 +142,9 @@ __global__ void wtc_output_kernel(const float *__restrict__ mm, Geometry q, OutA
             for(int j = 0; j < 2; j++) {
                 const int ox = 2 * tx + j;
                 if(ox >= q.w) continue;
-                const long long yi = (((long long)b * q.cout + o) * q.h + oy) * q.w + ox;
+                const long long yi = y0 + (long long)i * q.w + j;
                 float val = apply_act(out[j] + bias, a.act);
-                if(a.residual) val = apply_act(val + a.residual_scale * __ldg(a.residual + yi), a.post_act);
+                if(a.residual) val = apply_act(val + a.residual_scale * res[i][j], a.post_act);
                 if(a.factor != 0.0f) val += a.factor * a.y[yi];
                 a.y[yi] = val;
             }
