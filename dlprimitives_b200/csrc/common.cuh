@@ -99,8 +99,8 @@ __device__ __forceinline__ void pdl_wait()
 
 // Load of what a kernel before this one may have written.  A kernel that starts early is resident while that one writes, so these
 // are not the read-only loads (__ldg, pointers to const with __restrict__), which are for memory that nobody writes while the kernel
-// lives and which nothing holds behind pdl_wait().  Stores through pointers that may overlap hold plain loads back: a loop asks for
-// all that it reads before it stores.
+// lives and which nothing holds behind pdl_wait().  Stores through pointers that may overlap hold plain loads back: loops with many
+// of them ask for what they read before they store.
 template<typename T> __device__ __forceinline__ T ld_plain(const T *p) { return *p; }
 
 template<typename T> __host__ __device__ inline T ceil_div(T a, T b) { return (a + b - 1) / b; }

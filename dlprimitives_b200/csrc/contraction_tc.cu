@@ -876,9 +876,6 @@ __global__ void __launch_bounds__(256) split_finish_kernel(const Contraction p, 
         // the four rows follow each other in y when they are pixels of one image, or y is column-major
         const bool together = p.out_mode == OUT_COL_MAJOR || (p.out_mode == OUT_NCHW && p.plane % 4 == 0);
         const long long step = p.out_mode == OUT_ROW_MAJOR ? p.ldc : 1;
-        // bias, residual and old values of all four first: behind the first store their loads would go one after the other
-        long long at[4];
-        float out[4];
         #pragma unroll
         for(int j = 0; j < 4; j++) {
             if(row + j >= p.rows) break;
@@ -886,13 +883,7 @@ __global__ void __launch_bounds__(256) split_finish_kernel(const Contraction p, 
                 if(together || p.out_mode == OUT_ROW_MAJOR) r.out += step;
                 else r = make_row(p, row + j);
             }
-            at[j] = out_index(p, r, col);
-            out[j] = finish_output(p, r, row + j, col, a[j]);
-        }
-        #pragma unroll
-        for(int j = 0; j < 4; j++) {
-            if(row + j >= p.rows) break;
-            p.y[at[j]] = out[j];
+            p.y[out_index(p, r, col)] = finish_output(p, r, row + j, col, a[j]);
         }
     }
 }
