@@ -184,8 +184,10 @@ contraction_tf32x3_kernel(const float *packed, const Contraction p, int kblocks,
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh->tmem_base)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    if(MODE == A_GATHER || MODE == A_ROWTAPS)
+    if(MODE == A_GATHER || MODE == A_ROWTAPS) {
+        pdl_wait();                     // (every warp: the table is global memory too)
         for(int i = threadIdx.x; i < ktab_smem_entries / 2; i += NUM_THREADS) ktab_s[i] = __ldg(reinterpret_cast<const int4 *>(p.ktab) + i);
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();

@@ -38,6 +38,17 @@ def test_plain_loads(name):
     assert not found, found
 
 
+@pytest.mark.parametrize("name", [f for f in FILES if f.endswith(".cu")])
+def test_the_wait_comes_first(name):
+    """No kernel loads from global memory, the tables of a plan included, ahead of its first wait for the kernel before it."""
+    early = {k: v for k, v in kernels(code(name)).items() if "pdl_wait()" in v}
+    if "launch_pdl(" in code(name):
+        assert early
+    for kernel, text in early.items():
+        load = re.search(r"__ldg\(|ld_plain\(|ld_early\(|bulk_load\(|tma_load", text)
+        assert load is None or text.index("pdl_wait()") < load.start(), kernel
+
+
 def test_the_kernels_are_found():
     """The scan sees what it is meant to see."""
     seen = {k for f in FILES if f.endswith(".cu") for k in kernels(code(f))}
