@@ -155,11 +155,11 @@ struct TcBatch {
     int count = 1;
     long long a_stride = 0, y_stride = 0;
 };
-// Scratch that lets the launcher split K when the problem has too few tiles for the GPU (0: it would not split).
+// Scratch that lets the launcher split K as it likes best for any number of rows up to this one (0: it would split none of them).
 size_t tc_split_scratch_bytes(long long rows, const TcPacked &L);
 // Into how many parts a launch with this scratch (at any address) cuts K, and where in it the partial sums go; 1: not cut.
 int tc_split(long long rows, const TcPacked &L, void *scratch, size_t scratch_bytes, float **partial);
-// scratch may be null or short; the launcher then does not split.
+// scratch may be null or short; the launcher then does not split, or into fewer parts.
 dlp_status launch_contraction_tc(const Contraction &p, const TcPacked &L, const float *packed, cudaStream_t stream, void *scratch = nullptr,
                                  size_t scratch_bytes = 0, const TcBatch &batch = TcBatch());
 

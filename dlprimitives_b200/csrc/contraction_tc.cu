@@ -920,13 +920,14 @@ dlp_status tc_prepack(const TcPacked &L, const float *b, long long b_col_stride,
 }
 
 namespace {
-// How many equal parts to cut K into.  Time is counted in k-block periods (about 0.5 us): a CTA works through
+// How many equal parts to cut K into, at most max_parts.  Time is counted in k-block periods (about 0.5 us): a CTA works through
 // ceil(items / SMs) work items of (k-blocks per part + a fixed cost for pipeline fill and epilogue) each,
 // and a split run pays for the finishing kernel.  K is cut only when that model gains a tenth or more.
 // The constants are fitted to timings of batch-1 and batch-16 layer shapes with forced splits: 7 periods per work item; 3 for
 // the second launch, which starts under the first (3x3 512 -> 512 on 7x7, one image: 144 k-blocks 82 us, two parts 47, four 30,
 // eight 21), and its pass over the partial sums, written and read, at 2 MB a period.
-int choose_splits(long long rows, const TcPacked &L)
+constexpr int MAX_PARTS = 32;
+int choose_splits(long long rows, const TcPacked &L, int max_parts)
 {
     const long long tiles = ceil_div<long long>(rows, tc::BM) * (L.n_pad / L.bn);
     const int kb = L.k_pad / tc::BK, sms = sm_count();
@@ -935,7 +936,7 @@ int choose_splits(long long rows, const TcPacked &L)
     const double uncut = double(ceil_div<long long>(tiles, sms)) * (kb + item_fixed);
     int best = 1;
     double best_cost = 0.9 * uncut;
-    for(int s = 2; s <= 32 && kb / s >= 4; s++) {
+    for(int s = 2; s <= max_parts && kb / s >= 4; s++) {
         if(kb % s != 0) continue;
         const double cost = double(ceil_div<long long>(tiles * s, sms)) * (kb / s + item_fixed) + finish + per_part * (2 * s + 1);
         if(cost < best_cost) { best = s; best_cost = cost; }
@@ -1013,19 +1014,28 @@ static size_t split_bytes(long long rows, const TcPacked &L, int parts)
     return size_t(parts) * size_t(round_up<long long>(rows, tc::BM)) * L.n_pad * sizeof(float);
 }
 
+// Enough for every batch up to the planned one: a smaller one may want more parts (its partial sums are fewer bytes), and then more
+// bytes than the planned one.  Among row counts of as many tiles the smallest wants the most parts, so one of each is looked at.
 size_t tc_split_scratch_bytes(long long rows, const TcPacked &L)
 {
-    const int s = choose_splits(rows, L);
-    return s > 1 ? split_bytes(rows, L, s) + SPLIT_ALIGN : 0;
+    const long long tiles = std::min<long long>(ceil_div<long long>(rows, tc::BM), 4 * sm_count() / (L.n_pad / L.bn));
+    size_t most = 0;
+    for(long long t = 0; t < tiles; t++) {
+        const long long r = t * tc::BM + 1;
+        const int s = choose_splits(r, L, MAX_PARTS);
+        if(s > 1) most = std::max(most, split_bytes(r, L, s) + SPLIT_ALIGN);
+    }
+    return most;
 }
 
+// A scratch that is too short for the best number of parts takes fewer: the best of those that fit.
 int tc_split(long long rows, const TcPacked &L, void *scratch, size_t scratch_bytes, float **partial)
 {
     *partial = nullptr;
-    const int s = choose_splits(rows, L);
     const size_t skip = (SPLIT_ALIGN - reinterpret_cast<uintptr_t>(scratch) % SPLIT_ALIGN) % SPLIT_ALIGN;
-    if(s == 1 || scratch == nullptr || scratch_bytes < skip + split_bytes(rows, L, s)) return 1;
-    *partial = reinterpret_cast<float *>(static_cast<char *>(scratch) + skip);
+    if(scratch == nullptr || scratch_bytes <= skip) return 1;
+    const int s = choose_splits(rows, L, int(std::min<size_t>(MAX_PARTS, (scratch_bytes - skip) / split_bytes(rows, L, 1))));
+    if(s > 1) *partial = reinterpret_cast<float *>(static_cast<char *>(scratch) + skip);
     return s;
 }
 
@@ -1037,15 +1047,14 @@ dlp_status launch_contraction_tc(const Contraction &p, const TcPacked &L, const 
     if(batch.count > 65535) return fail(DLP_INVALID_ARGUMENT, "a batched product takes at most 65535 matrices");
     if(ceil_div<long long>(p.rows, tc::BM) * ceil_div(p.cols, L.bn) * batch.count >= (1ll << 31))
         return fail(DLP_INVALID_ARGUMENT, "more than 2^31 output tiles");
-    int splits = batch.count > 1 ? 1 : choose_splits(p.rows, L);      // the matrices of a batch fill the GPU between them
+    float *partial = nullptr;
+    const int splits = batch.count > 1 ? 1 : tc_split(p.rows, L, scratch, scratch_bytes, &partial);      // the matrices of a batch fill the GPU between them
     if(splits == 1 && batch.count == 1 && pointwise_tc_eligible(p, L)) return launch_pointwise_tc(p, L, packed, stream);
     // (environment variable DLP_TC_NO_STAGED: keep such problems on this file's kernel, for A/B timing and profiling)
     static const bool no_staged = getenv("DLP_TC_NO_STAGED") != nullptr;
     if(splits == 1 && batch.count == 1 && !no_staged && staged_tc_eligible(p, L)) return launch_staged_tc(p, L, packed, stream);
     const long long rows_pad = ceil_div<long long>(p.rows, tc::BM) * tc::BM;
     const long long split_stride = rows_pad * L.n_pad;
-    float *partial = nullptr;
-    if(splits > 1) splits = tc_split(p.rows, L, scratch, scratch_bytes, &partial);
     Contraction q = p;
     if(splits > 1) {
         // the parts write raw partial sums to the scratch; the epilogue runs in the finishing kernel

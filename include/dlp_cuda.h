@@ -83,7 +83,7 @@ DLP_API dlp_status dlp_tf32_issue_probe(int scheme, int n, double *cycles_per_kb
  * launches really use; needs no device. */
 DLP_API dlp_status dlp_pointwise_rings(int bn, int kblocks, int resident, int residual, int *a_slots, int *epilogue_buffers);
 /* Into how many parts a product of rows x cols with k terms is cut when it is called with this scratch, the bytes of scratch that
- * a plan for it asks for, and where in the scratch the partial sums go (offset in bytes).  A host-side rule; reads nothing through the
+ * a plan for as many rows asks for (enough for any smaller number, too), and where in the scratch the partial sums go (offset in bytes).  A host-side rule; reads nothing through the
  * pointer and needs no device. */
 DLP_API dlp_status dlp_split_rule(long long rows, int cols, int k, void *scratch, size_t scratch_bytes, int *parts, size_t *wanted_bytes,
                                   size_t *offset);
@@ -123,10 +123,10 @@ DLP_API void dlp_conv2d_fwd_destroy(dlp_conv2d_plan *plan);
 DLP_API const char *dlp_conv2d_fwd_algo(const dlp_conv2d_plan *plan);
 /* Name of the kernel variant behind the plan, e.g. "igemm_tf32x3_bn128". */
 DLP_API const char *dlp_conv2d_fwd_kernel(const dlp_conv2d_plan *plan);
-/* Conv2DBase::workspace(): bytes of scratch enqueue needs for the planned batch: the packed weights, plus,
+/* Conv2DBase::workspace(): bytes of scratch enqueue needs for the planned batch and any smaller one: the packed weights, plus,
  * for problems with too few output tiles to fill the GPU, room for partial sums over parts of K (the
  * results are added in a fixed order, so they do not depend on timing).  enqueue_packed uses a workspace
- * only for the latter, at any address; a short or missing one just turns the split off. */
+ * only for the latter, at any address; a short one means fewer parts, none turns the split off. */
 DLP_API size_t dlp_conv2d_fwd_workspace(const dlp_conv2d_plan *plan);
 /* Bytes of the pre-packed form of the weights (0 when the kernel reads raw weights). */
 DLP_API size_t dlp_conv2d_fwd_packed_bytes(const dlp_conv2d_plan *plan);
