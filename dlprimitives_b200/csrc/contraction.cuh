@@ -119,15 +119,20 @@ __device__ __forceinline__ long long out_index(const Contraction &p, const RowIn
     return p.out_mode == OUT_NCHW ? r.out + (long long)col * p.plane : (p.out_mode == OUT_COL_MAJOR ? r.out + (long long)col * p.ldc : r.out + col);
 }
 
+// activation, residual and old value of output idx, whose bias is in acc already
+__device__ __forceinline__ float finish_biased(const Contraction &p, long long idx, float acc)
+{
+    acc = apply_act(acc, p.act);
+    if(p.residual) acc = apply_act(acc + p.residual_scale * ld_plain(p.residual + idx), p.post_act);
+    if(p.beta != 0.0f) acc += p.beta * p.y[idx];
+    return acc;
+}
+
 __device__ __forceinline__ float finish_output(const Contraction &p, const RowInfo &r, long long row, int col, float acc)
 {
     if(p.bias_mode == DLP_GEMM_BIAS_N) acc += ld_plain(p.bias + col);
     else if(p.bias_mode == DLP_GEMM_BIAS_M) acc += ld_plain(p.bias + row);
-    acc = apply_act(acc, p.act);
-    long long idx = out_index(p, r, col);
-    if(p.residual) acc = apply_act(acc + p.residual_scale * ld_plain(p.residual + idx), p.post_act);
-    if(p.beta != 0.0f) acc += p.beta * p.y[idx];
-    return acc;
+    return finish_biased(p, out_index(p, r, col), acc);
 }
 
 // launchers (one per translation unit)

@@ -863,6 +863,8 @@ __global__ void __launch_bounds__(256) split_finish_kernel(const Contraction p, 
         const long long row = 4 * (long long)(idx - Index(col) * quads);
         const float *src = partial + (long long)col * rows_pad + row;
         float4 acc = ld_plain(reinterpret_cast<const float4 *>(src));
+        // (asked for with the partials: behind the first row's store it would be a trip of its own)
+        const float bias_n = p.bias_mode == DLP_GEMM_BIAS_N ? ld_plain(p.bias + col) : 0.0f;
         #pragma unroll 1
         for(int s = 1; s < splits; s += 8) {
             float4 v[8];
@@ -885,7 +887,9 @@ __global__ void __launch_bounds__(256) split_finish_kernel(const Contraction p, 
                 if(together || p.out_mode == OUT_ROW_MAJOR) r.out += step;
                 else r = make_row(p, row + j);
             }
-            p.y[out_index(p, r, col)] = finish_output(p, r, row + j, col, a[j]);
+            const long long at = out_index(p, r, col);
+            if(p.bias_mode == DLP_GEMM_BIAS_N) p.y[at] = finish_biased(p, at, a[j] + bias_n);
+            else p.y[at] = finish_output(p, r, row + j, col, a[j]);
         }
     }
 }
