@@ -54,6 +54,7 @@ SYMBOLS = {
     "dlp_last_error": (C.c_char_p, []),
     "dlp_version": (C.c_char_p, []),
     "dlp_launch_count": (C.c_uint64, []),
+    "dlp_last_route": (C.c_char_p, []),
     "dlp_device_status": (_i, [_vp, _ip]),
     "dlp_selftest_wait_expiry": (_i, [C.POINTER(C.c_int * 4), _vp]),
     "dlp_tf32_mma_rate": (_i, [C.POINTER(C.c_double), _vp]),
@@ -153,6 +154,12 @@ def _stream(stream=None):
 
 def launch_count():
     return int(lib().dlp_launch_count())
+
+
+def last_route():
+    """(kernel, column tile, parts of K) of this thread's last dense contraction."""
+    kernel, bn, parts = lib().dlp_last_route().decode().split()
+    return kernel, int(bn), int(parts)
 
 
 def device_status(stream=None):

@@ -22,6 +22,13 @@ dlp_status fail(dlp_status st, const std::string &msg)
     t_error = msg;
     return st;
 }
+static thread_local struct { const char *kernel = "none"; int bn = 0, parts = 0; } t_route;
+void note_route(const char *kernel, int bn, int parts)
+{
+    t_route.kernel = kernel;
+    t_route.bn = bn;
+    t_route.parts = parts;
+}
 dlp_status check_cuda(cudaError_t e, const char *what)
 {
     if(e == cudaSuccess) return DLP_OK;
@@ -100,6 +107,12 @@ extern "C" {
 const char *dlp_last_error(void) { return t_error.c_str(); }
 const char *dlp_version(void) { return "dlprim-b200 0.1 (sm_100a)"; }
 uint64_t dlp_launch_count(void) { return g_launches.load(); }
+const char *dlp_last_route(void)
+{
+    static thread_local std::string text;
+    text = std::string(t_route.kernel) + " " + std::to_string(t_route.bn) + " " + std::to_string(t_route.parts);
+    return text.c_str();
+}
 
 dlp_status dlp_device_status(void *stream, int *code)
 {

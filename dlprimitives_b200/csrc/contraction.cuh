@@ -140,6 +140,9 @@ __device__ __forceinline__ float finish_output(const Contraction &p, const RowIn
 dlp_status launch_contraction_ffma(const Contraction &p, int groups, long long a_group_stride, long long b_group_stride,
                                    int out_group_channels, cudaStream_t stream, long long y_group_stride = 0);
 
+// Notes what the calling thread's dense contraction is handed to (dlp_last_route); kernel: a literal.
+void note_route(const char *kernel, int bn, int parts);
+
 // Pre-packed B for the tensor-core kernel: zero padded and already split into its TF32 part (hi) and
 // the remainder (lo).  It is a sequence of pipeline stages in the order (column tile, k-block of 32);
 // a stage is the exact shared-memory image the kernel computes from -- the hi tile (bn rows of 32

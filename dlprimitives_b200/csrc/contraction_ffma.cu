@@ -102,6 +102,7 @@ dlp_status launch_contraction_ffma(const Contraction &p, int groups, long long a
                                    int out_group_channels, cudaStream_t stream, long long y_group_stride)
 {
     if(p.rows <= 0 || p.cols <= 0 || groups <= 0) return DLP_OK;
+    note_route("ffma", TN, 1);
     const long long gx = ceil_div<long long>(p.rows, TM);
     if(gx > 0x7fffffffLL) return fail(DLP_INVALID_ARGUMENT, "too many output rows for one launch");
     dim3 grid((unsigned)gx, (unsigned)ceil_div(p.cols, TN), (unsigned)groups);

@@ -974,6 +974,8 @@ dlp_status launch_bn(const Contraction &p, const TcPacked &L, const float *packe
     const long long m_tiles = ceil_div<long long>(p.rows, tc::BM);
     const int n_tiles = L.n_pad / BN;
     const long long num_tiles = m_tiles * n_tiles * splits;     // work items
+    note_route(MODE == A_GATHER ? "general_gather" : (MODE == A_STRIDED ? "general_strided" : (MODE == A_TAPBLOCK ? "general_taps" : "general_rowtaps")),
+               BN, splits);
     const dim3 grid(unsigned(std::min<long long>(num_tiles, sm_count())), unsigned(batch.count));
     int diag = 0;
     long long *trace = nullptr;

@@ -608,6 +608,7 @@ bool pointwise_tc_eligible(const Contraction &p, const TcPacked &L)
 
 dlp_status launch_pointwise_tc(const Contraction &p, const TcPacked &L, const float *packed, cudaStream_t stream)
 {
+    note_route("pointwise", L.bn, 1);
     const int images = int(p.rows / p.plane);
     CUtensorMap tx, ty, tr;
     dlp_status st = pw::make_map(tx, p.a, p.plane, p.k, p.a_batch_stride, images);

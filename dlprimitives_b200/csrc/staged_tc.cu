@@ -600,6 +600,7 @@ dlp_status launch_staged_tc(const Contraction &p, const TcPacked &L, const float
 {
     sg::Params q;
     if(!sg::plan(p, L, q)) return fail(DLP_INVALID_ARGUMENT, "not a problem for the staged convolution kernel");
+    note_route("staged", L.bn, 1);
     const int images = int(p.rows / p.plane);
     CUtensorMap tx, ty;
     {

@@ -770,6 +770,7 @@ dlp_status launch_stream_tc(const Contraction &p, const TcPacked &L, const float
     st::Source src;
     if(!st::plan(p, L, splits, batch, q, src)) return fail(DLP_INVALID_ARGUMENT, "not a problem for the streaming kernel");
     q.y_split_stride = split_stride;
+    note_route(src.kind == st::SRC_K ? "stream_k" : (src.kind == st::SRC_UNITS ? "stream_units" : "stream_copy"), L.bn, splits);
     CUtensorMap ta;
     memset(&ta, 0, sizeof(ta));
     if(src.kind != st::SRC_COPY) {

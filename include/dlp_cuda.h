@@ -55,6 +55,11 @@ DLP_API const char *dlp_version(void);
 /* Number of kernels this library has launched from the calling process so far (all threads). */
 DLP_API uint64_t dlp_launch_count(void);
 
+/* What the calling thread's last dense contraction (GEMM, InnerProduct, convolution but depthwise and fp32 Winograd) was handed to, as
+ * "kernel column-tile parts-of-K": general_{gather,strided,taps,rowtaps}, stream_{k,units,copy}, staged, pointwise, ffma.  For tests and
+ * timing; valid until the thread's next call of it. */
+DLP_API const char *dlp_last_route(void);
+
 /* The tensor-core kernels poll mbarriers with an iteration limit.  When a limit is hit the kernel
  * records a code in a per-device word, drains its copies, frees its tensor memory and returns.
  * This call synchronises `stream`, then reads and clears that word: 0 means no wait ever gave up. */
