@@ -68,10 +68,16 @@ inline cudaError_t launch_pdl(bool early, void (*kernel)(P...), dim3 grid, dim3 
     return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
-// blocks of a plain kernel (threads each, little shared memory) that are all resident at once
+// Blocks of a plain kernel (threads each) that are all resident at once as far as threads go; where registers or shared memory allow fewer
+// (global pooling's tiles, the banded depthwise kernel) it is a round or two more.  Captured chains of one layer, never early -> early
+// (us): depthwise 3x3 144x56x56 at 1, 4 and 8 images 4.0 -> 3.6, 5.9 -> 5.5, 9.1 -> 8.7, 960x7x7 at 32 8.2 -> 7.9; beyond the line no
+// difference to speak of (96x112x112 and 960x7x7 at 128: within 0.2), and behind other kernels a loss (above).
 inline bool one_wave(long long blocks, int threads) { return blocks * threads <= (long long)sm_count() * 2048; }
-// work items of a persistent tensor-core kernel that are few enough for the set-up to matter (3x3 64 -> 64 on 56x56 at batch 16, 448
-// items, with the packing of its weights before it: 43.0 us in stream order, 40.3 us started early)
+// Work items of a persistent tensor-core kernel that are few enough for the set-up to matter.  Captured chains of one layer, never
+// early -> early (us): 3x3 64 -> 64 on 56x56 at batch 4, 16 and 21 (112, 448 and 588 items) 14.2 -> 13.1, 36.8 -> 34.6, 36.9 -> 35.5;
+// 3x3 128 -> 128 on 28x28 at 16 27.3 -> 25.8; 1x1 64 -> 256 on 56x56 with residual at 4 and 11 13.6 -> 12.6, 19.2 -> 18.2; 1x1 256 ->
+// 1024 on 14x14 with residual at 16 and 32 18.9 -> 17.5, 25.5 -> 24.7, but at 48 (592 items) 34.8 -> 36.5.  Further on a chain of one
+// layer would still gain up to 2 us (batch 22 to 48 of the first), a network of different layers loses (above).
 inline bool few_items(long long items) { return items <= 4ll * sm_count(); }
 
 // ---- device side ---------------------------------------------------------------------------------

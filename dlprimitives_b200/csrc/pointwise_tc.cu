@@ -12,7 +12,7 @@
 //       - B (packed weights): with few input channels the whole column tile's weights fit in shared memory and
 //         a CTA works on one column tile throughout, so they are copied once per CTA and stay; otherwise they
 //         stream through a ring, one bulk copy per k-block.
-//       - residual operand: a tensor-map copy per 32 channels of the tile into one of three epilogue buffers,
+//       - residual operand: a tensor-map copy per 32 channels of the tile into one of the epilogue buffers,
 //         issued by its own thread as soon as a buffer is free (up to two groups ahead of the epilogue warps).
 //       - result: the epilogue warps read the accumulator from tensor memory, add bias / activation / residual,
 //         write the finished 128 x 32 block into the same epilogue buffer and one thread stores it with a

@@ -29,11 +29,13 @@
 //     leaves, and tensor memory is freed on every path.
 //
 // What bounds it now is shared memory: per k-block of 128 columns the MMAs read 48 KB of weights (hi twice, lo once), the copies
-// write 32 KB of weights and 16 KB (3 KB with nine taps) of A, and the converters read 16 KB: 112 KB at 128 bytes a cycle are 875
+// write 32 KB of weights and 16 KB (3 KB with nine taps) of A, and the converters read 16 KB: 112 KB at 128 bytes a cycle are 896
 // cycles, and 1040 are measured (tensor pipe 75 % active on 4096 x 4096 x 4096; the SM clock then settles at 1.6 GHz).
-// Measured against the general kernel, same process (us): 2048^3 A * B^T 139 -> 95, A^T * B^T 113 -> 101, 4096^3 913 -> 620,
-// InnerProduct 4096 -> 4096 on 1024 rows 234 -> 161, 2048 -> 1000 on 256 rows 37 -> 28, on one row 31 -> 23; 3x3 128 -> 128 on 28x28 at
-// batch 256 247 -> 243, 5x5 64 -> 192 on 28x28 at batch 64 231 -> 202.
+// Measured against the general kernel, as whole calls (us): before this kernel and with it, 2048^3 A * B^T with the packing of B 134 -> 98.5,
+// InnerProduct 2048 -> 1000 on 256 rows of raw weights 38.9 -> 25.1 and on one row of packed ones 24.6 -> 14.9 (launches that start early
+// and a cheaper finishing pass are in both); calls captured one after the other, A as it is and four bytes off a 16-byte boundary,
+// which is the general kernel's with single loads: 2048^3 A^T * B^T 90 against 107, InnerProduct 2048 -> 1000 on one row 14.7 against
+// 17.5, 3x3 128 -> 128 on 28x28 at batch 256 271 against 277, 256 -> 256 on 14x14 283 against 285.
 //
 // Reference: the implicit GEMM and the plain GEMM of src/kernels/sgemm.cl:71-134.
 #define DLP_INLINE_WAITS
@@ -64,6 +66,8 @@ constexpr int NUM_WARPS = 20, NUM_THREADS = NUM_WARPS * 32;
 // Registers per thread of the warpgroups after the split (launched with 96): copies and issue 40, accumulate 128 (64 sums), convert 88:
 // 40 + 2 * 128 + 2 * 88 = 472 of 5 * 96 = 480.
 constexpr int REGS_LAUNCH = 96, REGS_ISSUE = 40, REGS_ACC = 128, REGS_CONV = 88;
+// 96 at launch are what 640 threads leave each.  With units and copies the 128-column kernels spill 60 bytes a thread (88 loaded), the
+// narrower ones 20 to 40; with K-major A the 128-column one 32 (64).
 static_assert(REGS_ISSUE + 2 * REGS_ACC + 2 * REGS_CONV <= 5 * REGS_LAUNCH, "setmaxnreg draws on the launch's registers");
 constexpr int SMEM_LIMIT = 227 * 1024;
 constexpr int SMEM_FIXED = 1024 + 1024;     // alignment slack + the barrier block and tables (+ a unit of zeros when there are taps)
@@ -93,7 +97,7 @@ struct Params {
     int P;                  // rows per image (the whole matrix when there are no images)
     int W, H;               // input plane of a convolution with taps
     int taps;               // k-blocks per slot (1: no halo, no masks)
-    int kh, kw, dil_h, dil_w, pad_h, pad_w;
+    int kw, dil_h, dil_w, pad_h, pad_w;
     int dmin, dmax;         // smallest and largest displacement of a tap in pixels
     int kblocks;            // k-blocks per work item
     int kblocks_all;        // of the whole K (work items of a split K take equal parts)
@@ -664,7 +668,7 @@ static bool plan(const Contraction &p, const TcPacked &L, int splits, const TcBa
         q.W = p.in_w;
         q.H = p.in_h;
         q.taps = p.num_taps;
-        q.kh = p.kh; q.kw = p.kw; q.dil_h = p.dil_h; q.dil_w = p.dil_w; q.pad_h = p.pad_h; q.pad_w = p.pad_w;
+        q.kw = p.kw; q.dil_h = p.dil_h; q.dil_w = p.dil_w; q.pad_h = p.pad_h; q.pad_w = p.pad_w;
         if(q.taps < 2 || q.taps > MAX_TAPS || q.taps != p.kh * p.kw || p.k % (q.taps * BK) != 0) return false;
         if(2 * p.pad_h != p.dil_h * (p.kh - 1) || 2 * p.pad_w != p.dil_w * (p.kw - 1)) return false;
         if(q.kblocks % q.taps != 0) return false;                       // a part of a split K is whole channel blocks
