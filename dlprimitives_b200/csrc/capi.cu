@@ -251,6 +251,9 @@ dlp_status dlp_conv2d_fwd_create(const dlp_conv2d_desc *desc, dlp_conv2d_plan **
             cudaError_t e = cudaMalloc((void **)&plan->tap_dydx, sizeof(int) * taps.size());
             if(e == cudaSuccess) e = cudaMemcpy(plan->ktab, tab.data(), sizeof(KTap) * k_pad, cudaMemcpyHostToDevice);
             if(e == cudaSuccess) e = cudaMemcpy(plan->tap_dydx, taps.data(), sizeof(int) * taps.size(), cudaMemcpyHostToDevice);
+            // A copy from pageable memory may return with its last part still on the way; a launch on any stream reads the tables at once,
+            // some of them (contraction_tf32x3_kernel) ahead of stream order.
+            if(e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
             if(e != cudaSuccess) {
                 cudaFree(plan->ktab);
                 if(plan->tap_dydx) cudaFree(plan->tap_dydx);

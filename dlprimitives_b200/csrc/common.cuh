@@ -46,7 +46,7 @@ int sm_count();
 // Launch of a kernel of the path.  `early`: it may start while the kernel before it on the stream is still running
 // (programmatic dependent launch): its blocks are set up -- and wait in pdl_wait() -- under the other's last blocks instead of
 // after them.  The waiting is the kernel's own: every kernel launched this way calls pdl_wait() in each thread before its first
-// access to global memory, and before its first wait for another warp: those waits are limited in time, and the kernel before
+// access to global memory (but for the index tables of a plan, which no kernel writes), and before its first wait for another warp: those waits are limited in time, and the kernel before
 // may take longer than the limit.  A kernel or copy of somebody else's before or after it is ordered in full as ever.
 // For launches whose blocks all fit on the GPU at once (one_wave): there the set-up is a good part of the time (InnerProduct
 // 2048 -> 1000 on one row 24.6 -> 21.3 us, on 256 rows with its packing 38.9 -> 33.3 us).  Longer launches lose more than
