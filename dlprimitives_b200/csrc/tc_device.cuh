@@ -207,12 +207,12 @@ __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&v)[32])
 }
 __host__ __device__ __forceinline__ bool act_is_clamp(int act) { return act == DLP_ACT_IDENTITY || act == DLP_ACT_RELU || act == DLP_ACT_RELU6; }
 // Bounds of an activation that is a clamp, fminf(fmaxf(v, .x), .y), with a NaN treated as in apply_act: relu and relu6 make it 0, the
-// identity keeps it.  The identity's bounds are NaN: of a number and a NaN, fmaxf and fminf give the number, of two NaNs a NaN
+// identity keeps it.  A bound that is not there is NaN: of a number and a NaN, fmaxf and fminf give the number, of two NaNs a NaN
 // (bounds of -inf and inf would turn a NaN into -inf).
 __device__ __forceinline__ float2 act_clamp(int act)
 {
     const float none = __int_as_float(0x7fffffff);
-    return make_float2(act == DLP_ACT_IDENTITY ? none : 0.0f, act == DLP_ACT_RELU6 ? 6.0f : (act == DLP_ACT_IDENTITY ? none : INFINITY));
+    return make_float2(act == DLP_ACT_IDENTITY ? none : 0.0f, act == DLP_ACT_RELU6 ? 6.0f : none);
 }
 
 // ---- tensor-map (TMA) copies of one box of a 3-D tensor; the map lives in kernel parameter space
